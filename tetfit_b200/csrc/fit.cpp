@@ -28,7 +28,7 @@ void fit_launch_step(const FitGrid<T>& g, const SpecialEdges<T>& sp, const Probe
                      const FitLoss<T>* loss, const FitTmaMaps* tma);
 bool fit_make_tma_maps(void* const U[3], void* const F[3], int es, int Nx, int Ny, int Nz, int64_t sx,
                        FitTmaMaps* out);
-int fit_kernels_per_step(int n_special, int n_probes, bool losses);
+int fit_kernels_per_step(int n_special, int n_probes, bool losses, bool classes);
 size_t fit_loss_parts(int Nx, int Ny, int Nz);
 template <typename T>
 size_t fit_launch_energy(const FitGrid<T>& g, double* part, cudaStream_t st);
@@ -803,7 +803,7 @@ void FitSim::fill_grid(FitGrid<T>& g, SpecialEdges<T>& s) {
   g.Fx = (T*)dF_[0]; g.Fy = (T*)dF_[1]; g.Fz = (T*)dF_[2];
   g.mat = dmat_;
   g.Nx = Nx_; g.Ny = Ny_; g.Nz = Nz_;
-  g.sx = sx_; g.sxy = sxy_;
+  g.sx = sx_; g.sxy = sxy_; g.nslot = nslot_;
   g.dt = dt_;
   g.P = dP_; g.S = dS_; g.R = dR_; g.X = dX_;
   g.mh_pure = (const T*)dmh_; g.mq_pure = (const T*)dmq_; g.mnu_pure = (const T*)dmnu_; g.mmu_pure = (const T*)dmmu_;
@@ -830,6 +830,24 @@ void FitSim::fill_grid(FitGrid<T>& g, SpecialEdges<T>& s) {
   s.flux_part = dflux_part_;
 }
 
+void* FitSim::dalloc(size_t bytes) {
+  void* p = nullptr;
+  if (bytes == 0) bytes = 16;
+  CU(cudaMalloc(&p, bytes));
+  allocs_.push_back(p);
+  dev_bytes_ += bytes;
+  return p;
+}
+
+// per-dof coefficient arrays of kernel variant 3
+void FitSim::alloc_coefficients() {
+  const size_t es = opt_.precision == 1 ? sizeof(float) : sizeof(double);
+  for (int q = 0; q < 12; q++) {
+    dC_[q] = dalloc(nslot_ * es);
+    CU(cudaMemsetAsync(dC_[q], 0, nslot_ * es, stream_));
+  }
+}
+
 void FitSim::alloc_device() {
   CU(cudaSetDevice(opt_.device));
   int major = 0;
@@ -839,40 +857,31 @@ void FitSim::alloc_device() {
   CU(cudaEventCreate(&ev0_));
   CU(cudaEventCreate(&ev1_));
   const size_t es = opt_.precision == 1 ? sizeof(float) : sizeof(double);
-  auto dalloc = [&](size_t bytes) -> void* {
-    void* p = nullptr;
-    if (bytes == 0) bytes = 16;
-    CU(cudaMalloc(&p, bytes));
-    allocs_.push_back(p);
-    dev_bytes_ += bytes;
-    return p;
-  };
-  for (int a = 0; a < 3; a++) {
-    dU_[a] = dalloc(nslot_ * es);
-    dF_[a] = dalloc(nslot_ * es);
-    CU(cudaMemsetAsync(dU_[a], 0, nslot_ * es, stream_));
-    CU(cudaMemsetAsync(dF_[a], 0, nslot_ * es, stream_));
-  }
+  // the class kernels read the neighbours of every slot: a zeroed plane and a
+  // row more before and after the slots (strides and so the pad are multiples
+  // of 8 slots, which keeps the arrays' 16-byte alignment)
+  const int64_t pad = sxy_ + sx_;
+  for (int a = 0; a < 3; a++)
+    for (void** p : {&dU_[a], &dF_[a]}) {
+      const size_t bytes = (size_t)(nslot_ + 2 * pad) * es;
+      char* base = (char*)dalloc(bytes);
+      CU(cudaMemsetAsync(base, 0, bytes, stream_));
+      *p = base + pad * es;
+    }
   dmat_ = (uint8_t*)dalloc(mat_.size());
   const size_t nm3 = 3 * mat_label_.size();
   dP_ = (double*)dalloc(nm3 * 8); dS_ = (double*)dalloc(nm3 * 8);
   dR_ = (double*)dalloc(nm3 * 8); dX_ = (double*)dalloc(nm3 * 8);
   dmh_ = dalloc(nm3 * es); dmq_ = dalloc(nm3 * es); dmnu_ = dalloc(nm3 * es); dmmu_ = dalloc(nm3 * es);
   dlive_ = (uint8_t*)dalloc(mat_label_.size());
-  dstep_ = (int*)dalloc(sizeof(int));
-  if (opt_.fit_variant == 4 || (opt_.fit_variant == 0 && n_cells() >= 2000000))
-    // the per-dof coefficient variant is forced or among the autotuner's candidates
-    for (int q = 0; q < 12; q++) {
-      dC_[q] = dalloc(nslot_ * es);
-      CU(cudaMemsetAsync(dC_[q], 0, nslot_ * es, stream_));
-    }
-  if (opt_.fit_variant == 6 || (opt_.fit_variant == 0 && n_cells() >= 2000000)) {
-    // the coefficient-class variant is forced or among the autotuner's candidates
+  dstep_ = (int*)dalloc(2 * sizeof(int));
+  if (opt_.fit_variant == 4) alloc_coefficients();
+  if (opt_.fit_variant == 6 || opt_.fit_variant == 0) {
     for (int q = 0; q < 6; q++) {
       dK_[q] = (uint16_t*)dalloc(nslot_ * sizeof(uint16_t));
-      CU(cudaMemsetAsync(dK_[q], 0, nslot_ * sizeof(uint16_t), stream_));
+      CU(cudaMemsetAsync(dK_[q], 0xff, nslot_ * sizeof(uint16_t), stream_));
     }
-    for (int q = 0; q < 2; q++) dlut_[q] = dalloc((size_t)2 * kMaxClasses * es);
+    for (int q = 0; q < 2; q++) dlut_[q] = dalloc((size_t)2 * (kMaxClasses + 1) * es);
   }
   dflux_ = (double*)dalloc(nsteps_ * 8);
   // Joule losses (Discretization.hpp:1902): the reference's Si is non-zero
@@ -910,6 +919,7 @@ void FitSim::alloc_device() {
   dinvmu_ = (double*)dalloc(3 * np * 8);
   dslot_ = (int*)dalloc(nsteps_ * 4);
   dsamples_ = (double*)dalloc((size_t)nslots_ * np * 6 * 8);
+  dpfaces_ = dalloc(6 * np * es);
   // tensor maps of the TMA z-march (variant 4) and its wait-timeout flag
   dtma_err_ = (int*)dalloc(sizeof(int));
   CU(cudaMemsetAsync(dtma_err_, 0, sizeof(int), stream_));
@@ -1121,19 +1131,25 @@ void FitSim::upload() {
 // coefficient classes of the class variant, from the same tables and
 // functions as the table-driven kernels (bit-identical).
 void FitSim::build_coefficients() {
-  if (dC_[0]) {
-    if (opt_.precision == 1) {
-      FitGrid<float> g; SpecialEdges<float> s;
-      fill_grid(g, s);
-      CU(fit_build_coefficients<float>(g, stream_));
-    } else {
-      FitGrid<double> g; SpecialEdges<double> s;
-      fill_grid(g, s);
-      CU(fit_build_coefficients<double>(g, stream_));
-    }
-    CU(cudaStreamSynchronize(stream_));
+  if (dK_[0]) build_classes();
+  if (opt_.fit_variant == 0 && cls_ok_) e_var_ = h_var_ = 5;
+  // more classes than the tables hold, on a grid the autotuner measures: the
+  // arrays are among its candidates
+  if (opt_.fit_variant == 0 && !cls_ok_ && n_cells() >= 2000000) alloc_coefficients();
+  if (!dC_[0]) return;
+  if (opt_.precision == 1) {
+    FitGrid<float> g; SpecialEdges<float> s;
+    fill_grid(g, s);
+    CU(fit_build_coefficients<float>(g, stream_));
+  } else {
+    FitGrid<double> g; SpecialEdges<double> s;
+    fill_grid(g, s);
+    CU(fit_build_coefficients<double>(g, stream_));
   }
-  if (!dK_[0]) return;
+  CU(cudaStreamSynchronize(stream_));
+}
+
+void FitSim::build_classes() {
   // hash tables of the build: set-up only, released before stepping
   FitClassWork w{};
   void* work = nullptr;
@@ -1149,11 +1165,11 @@ void FitSim::build_coefficients() {
   if (opt_.precision == 1) {
     FitGrid<float> g; SpecialEdges<float> s;
     fill_grid(g, s);
-    e = fit_build_classes<float>(g, w, ncls, stream_);
+    e = fit_build_classes<float>(g, s, w, ncls, stream_);
   } else {
     FitGrid<double> g; SpecialEdges<double> s;
     fill_grid(g, s);
-    e = fit_build_classes<double>(g, w, ncls, stream_);
+    e = fit_build_classes<double>(g, s, w, ncls, stream_);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
   cudaFree(work);
@@ -1164,10 +1180,11 @@ void FitSim::build_coefficients() {
 }
 
 void FitSim::launch_steps(int n, cudaEvent_t* ev) {
+  tma_used_ = tma_used_ || e_var_ == 4 || h_var_ == 4;
   ProbeSet pr;
   pr.n = (int)probe_cell_.size();
   pr.ci = dpi_; pr.cj = dpj_; pr.ck = dpk_;
-  pr.inv_mu = dinvmu_; pr.samples = dsamples_; pr.slot_of_step = dslot_;
+  pr.inv_mu = dinvmu_; pr.samples = dsamples_; pr.slot_of_step = dslot_; pr.faces = dpfaces_;
   if (opt_.precision == 1) {
     FitGrid<float> g; SpecialEdges<float> s;
     fill_grid(g, s);
@@ -1186,9 +1203,13 @@ void FitSim::launch_steps(int n, cudaEvent_t* ev) {
   }
 }
 
-// Project autotuner: on grids of at least 2 M cells the first steps of a run
-// cycle through the E and H kernel variants (bit-identical results), timing
-// each with events, and keep the fastest of each for the rest of the run.
+// Kernel variant of a run.  Coefficient classes whenever the tables hold the
+// scene's classes: two launches a step against five, and the fastest E and H
+// of all variants at every size measured (FP32 and FP64, 24^3 to 512^3).
+// Otherwise the 16-plane z-march, and on grids of at least 2 M cells the
+// project autotuner: the first steps of the run cycle through the remaining E
+// and H variants (bit-identical results), timing each with events, and keep
+// the fastest of each for the rest of the run.
 void FitSim::autotune(uint64_t& n) {
   if (opt_.fit_variant > 0) {
     e_var_ = h_var_ = opt_.fit_variant - 1;
@@ -1198,13 +1219,12 @@ void FitSim::autotune(uint64_t& n) {
     tuned_ = true;
     return;
   }
-  if (tuned_ || n_cells() < 2000000) { tuned_ = true; return; }
-  // candidates: node slot, 4- and 16-plane z-march, per-dof coefficients
-  // (when allocated), TMA z-march (when the tensor maps exist), coefficient
-  // classes (when the tables were built)
-  int cand[6], kVariants = 0;
-  for (int v = 0; v < 6; v++)
-    if ((v != 3 || dC_[0]) && (v != 4 || tma_ok_) && (v != 5 || cls_ok_)) cand[kVariants++] = v;
+  if (tuned_ || cls_ok_ || n_cells() < 2000000) { tuned_ = true; return; }
+  // candidates: node slot, 4- and 16-plane z-march, per-dof coefficients,
+  // TMA z-march (when the tensor maps exist)
+  int cand[5], kVariants = 0;
+  for (int v = 0; v < 5; v++)
+    if ((v != 3 || dC_[0]) && (v != 4 || tma_ok_)) cand[kVariants++] = v;
   const int kReps = 2;
   cudaEvent_t ev[6];
   for (auto& e : ev) CU(cudaEventCreate(&e));
@@ -1264,6 +1284,7 @@ uint64_t FitSim::step(uint64_t n) {
   CU(cudaEventRecord(ev0_, stream_));
   uint64_t left = n;
   if (glen > 1 && graph_ && graph_len_ == glen) {
+    tma_used_ = tma_used_ || e_var_ == 4 || h_var_ == 4;
     while (left >= (uint64_t)glen) {
       CU(cudaGraphLaunch(graph_, stream_));
       left -= glen;
@@ -1283,7 +1304,8 @@ uint64_t FitSim::step(uint64_t n) {
 
 // A TMA march whose mbarrier wait gave up leaves the step's results invalid.
 void FitSim::check_tma() {
-  if (!tma_ok_) return;
+  if (!tma_used_) return;
+  tma_used_ = false;
   int e = 0;
   CU(cudaMemcpy(&e, dtma_err_, sizeof(int), cudaMemcpyDeviceToHost));
   if (!e) return;
@@ -1292,7 +1314,7 @@ void FitSim::check_tma() {
 }
 
 int FitSim::kernels_per_step() const {
-  return fit_kernels_per_step((int)special_.size(), (int)probe_cell_.size(), losses_on_);
+  return fit_kernels_per_step((int)special_.size(), (int)probe_cell_.size(), losses_on_, e_var_ == 5 && h_var_ == 5);
 }
 
 // Per-phase device time over n steps (sources/BC, E, scatter+flux, probes, H),

@@ -147,20 +147,24 @@ class FitSim : public Sim {
   // probes
   int *dpi_ = nullptr, *dpj_ = nullptr, *dpk_ = nullptr, *dslot_ = nullptr;
   double *dinvmu_ = nullptr, *dsamples_ = nullptr;
+  void* dpfaces_ = nullptr;   // the probe cells' face values before the H half
   double* pinned_ = nullptr;  // host staging for step_io
   int e_var_ = 2, h_var_ = 2; // kernel variants (see fit_launch_step)
   bool tuned_ = false;
   int tune_pos_ = 0;
-  double tune_e_[6] = {0, 0, 0, 0, 0, 0}, tune_h_[6] = {0, 0, 0, 0, 0, 0};
+  double tune_e_[5] = {0, 0, 0, 0, 0}, tune_h_[5] = {0, 0, 0, 0, 0};
   FitTmaMaps tma_{};
-  bool tma_ok_ = false;
+  bool tma_ok_ = false, tma_used_ = false;
   int* dtma_err_ = nullptr;
-  void* dC_[12] = {};  // per-dof coefficients M_h, M_q, M_nu, M_mu x 3 axes (autotuned grids)
+  void* dC_[12] = {};  // per-dof coefficients M_h, M_q, M_nu, M_mu x 3 axes (variant 3)
   uint16_t* dK_[6] = {};  // coefficient classes of the x, y, z edges, then faces
   void* dlut_[2] = {};    // class tables (edges, faces)
   bool cls_ok_ = false;
   int ncls_[2] = {0, 0};  // edge and face classes (-1: more than the tables hold)
   void build_coefficients();
+  void build_classes();
+  void* dalloc(size_t bytes);
+  void alloc_coefficients();
 
  public:
   int kernel_variant() const override { return e_var_ + 8 * h_var_; }

@@ -747,71 +747,98 @@ __device__ __forceinline__ T* comp_ptr(T* x, T* y, T* z, int c) {
   return c == 0 ? x : (c == 1 ? y : z);
 }
 
-// Special edges: new values into sp.out, flux partial sums per block.
-template <typename T>
-__global__ void __launch_bounds__(256) fit_special_pre(FitGrid<T> g, SpecialEdges<T> sp, const int* step_counter) {
+// Special edges of block b: new values into sp.out (or, with kDirect, into
+// U), flux partial sums per block.
+template <typename T, bool kDirect, bool kPdl>
+__device__ __forceinline__ void special_edges(const FitGrid<T>& g, const SpecialEdges<T>& sp,
+                                              const int* step_counter, int b) {
   using A = Ar<T>;
   __shared__ double red[256];
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  const int step = *step_counter;
+  const int e = b * 256 + threadIdx.x;
   double contrib = 0.0;
+  // the edge's tables, its first source's among them, before the fields
+  int64_t slot = 0, fs[4] = {0, 0, 0, 0};
+  int op = 0, nf = 0, comp = 0, p0 = 0, p1 = 0, si0 = 0, d0 = 0;
+  int fc[4] = {0, 0, 0, 0};
+  double amp0 = 0.0, f0[4] = {0.0, 0.0, 0.0, 0.0}, w[3] = {0.0, 0.0, 0.0}, post = 0.0, cmh = 0.0, cmq = 0.0;
+  T sg[4] = {0, 0, 0, 0};
   if (e < sp.n) {
-    T* U = comp_ptr(g.Ux, g.Uy, g.Uz, sp.comp[e]);
-    const int64_t slot = sp.slot[e];
+    p0 = sp.src_begin[e];
+    p1 = sp.src_begin[e + 1];
+    slot = sp.slot[e];
+    comp = sp.comp[e];
+    op = sp.op[e];
+    nf = sp.nface[e];
+    cmh = sp.mh[e];
+    cmq = sp.mq[e];
+    post = sp.post[e];
+#pragma unroll
+    for (int q = 0; q < 3; q++) w[q] = sp.pair_vec[3 * (int64_t)e + q];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      fs[q] = sp.fslot[4 * e + q];
+      fc[q] = sp.fcomp[4 * e + q];
+      sg[q] = (T)sp.fsign[4 * e + q];
+    }
+    if (p0 < p1) {
+      si0 = sp.pair_src[p0];
+      d0 = sp.pair_dir[p0];
+#pragma unroll
+      for (int q = 0; q < 4; q++) f0[q] = sp.pair_fac[4 * p0 + q];
+      amp0 = sp.src_amp[si0];
+    }
+  }
+  if (kPdl) cudaGridDependencySynchronize();
+  const int step = *step_counter;
+  if (e < sp.n) {
+    T* U = comp_ptr(g.Ux, g.Uy, g.Uz, comp);
     const T Uo = U[slot];
     // source value: sum of source vectors, dotted with the projection vector
-    double v[3] = {0.0, 0.0, 0.0};
+    double v0 = 0.0, v1 = 0.0, v2 = 0.0;
     int kind = 0;
-    for (int p = sp.src_begin[e]; p < sp.src_begin[e + 1]; p++) {
-      const int si = sp.pair_src[p];
+    for (int p = p0; p < p1; p++) {
+      const int si = p == p0 ? si0 : sp.pair_src[p];
       kind = sp.src_kind[si] + 1;
-      double ret = __dmul_rn(sp.src_amp[si], sp.carrier[(int64_t)step * sp.nsrc + si]);
-      ret = __dmul_rn(ret, sp.pair_fac[4 * p + 0]);
-      ret = __dmul_rn(ret, sp.pair_fac[4 * p + 1]);
-      ret = __dmul_rn(ret, sp.pair_fac[4 * p + 2]);
-      ret = __dmul_rn(ret, sp.pair_fac[4 * p + 3]);
-      const int d = sp.pair_dir[p];
-      v[d] = __dadd_rn(v[d], ret);
+      double ret = __dmul_rn(p == p0 ? amp0 : sp.src_amp[si], sp.carrier[(int64_t)step * sp.nsrc + si]);
+#pragma unroll
+      for (int q = 0; q < 4; q++) ret = __dmul_rn(ret, p == p0 ? f0[q] : sp.pair_fac[4 * p + q]);
+      const int d = p == p0 ? d0 : sp.pair_dir[p];
+      if (d == 0) v0 = __dadd_rn(v0, ret);
+      else if (d == 1) v1 = __dadd_rn(v1, ret);
+      else v2 = __dadd_rn(v2, ret);
     }
     double val = 0.0;
     if (kind) {
-      const double* w = sp.pair_vec + 3 * (int64_t)e;
-      val = __dadd_rn(__dadd_rn(__dmul_rn(v[0], w[0]), __dmul_rn(v[1], w[1])), __dmul_rn(v[2], w[2]));
-      val = __dmul_rn(sp.post[e], val);
+      val = __dadd_rn(__dadd_rn(__dmul_rn(v0, w[0]), __dmul_rn(v1, w[1])), __dmul_rn(v2, w[2]));
+      val = __dmul_rn(post, val);
     }
-    const int op = sp.op[e];
     T Un;
     if (op == 0) {
       Un = kind == 1 ? (T)val : (T)0;
     } else {
       const T dt = (T)g.dt;
       T f[4];
-      const int nf = sp.nface[e];
-      for (int q = 0; q < 4; q++) {
-        f[q] = (T)0;
-        if (q < nf) {
-          const T* F = comp_ptr(g.Fx, g.Fy, g.Fz, sp.fcomp[4 * e + q]);
-          f[q] = F[sp.fslot[4 * e + q]];
-        }
-      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) f[q] = q < nf ? comp_ptr(g.Fx, g.Fy, g.Fz, fc[q])[fs[q]] : (T)0;
       const T I = kind == 3 ? (T)val : (T)0;
-      const T mh = (T)sp.mh[e], mq = (T)sp.mq[e];
+      const T mh = (T)cmh, mq = (T)cmq;
       T cf;
       if (op == 1) {  // explicit signed faces, Eigen 3-vector dot order
-        T acc = A::add(A::mul(f[0], (T)sp.fsign[4 * e]), A::mul(f[1], (T)sp.fsign[4 * e + 1]));
-        acc = A::add(acc, A::mul(f[2], (T)sp.fsign[4 * e + 2]));
-        if (nf > 3) acc = A::add(acc, A::mul(f[3], (T)sp.fsign[4 * e + 3]));
+        T acc = A::add(A::mul(f[0], sg[0]), A::mul(f[1], sg[1]));
+        acc = A::add(acc, A::mul(f[2], sg[2]));
+        if (nf > 3) acc = A::add(acc, A::mul(f[3], sg[3]));
         const T cfb = kind == 2 ? (T)val : (T)0;
         cf = A::sub(A::add(acc, cfb), I);
         Un = A::mul(mh, A::add(A::mul(mq, Uo), A::mul(dt, cf)));
         contrib = __dmul_rn(__dadd_rn((double)Uo, (double)Un), (double)cfb);
       } else {  // interior stencil with a dipole current
         T st = A::sub(A::add(A::sub(f[0], f[1]), f[2]), f[3]);
-        cf = A::sub(A::mul((T)sp.fsign[4 * e], st), I);
+        cf = A::sub(A::mul(sg[0], st), I);
         Un = A::mul(mh, A::add(A::mul(mq, Uo), A::mul(dt, cf)));
       }
     }
-    sp.out[e] = Un;
+    if (kDirect) U[slot] = Un;
+    else sp.out[e] = Un;
   }
   red[threadIdx.x] = contrib;
   __syncthreads();
@@ -819,7 +846,26 @@ __global__ void __launch_bounds__(256) fit_special_pre(FitGrid<T> g, SpecialEdge
     if (threadIdx.x < w) red[threadIdx.x] = __dadd_rn(red[threadIdx.x], red[threadIdx.x + w]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) sp.flux_part[blockIdx.x] = red[0];
+  if (threadIdx.x == 0) sp.flux_part[b] = red[0];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) fit_special_pre(FitGrid<T> g, SpecialEdges<T> sp, const int* step_counter) {
+  special_edges<T, false, false>(g, sp, step_counter, blockIdx.x);
+}
+
+// Fixed-order sum of a step's flux partials (one block).
+__device__ __forceinline__ void flux_total(const double* part, int nparts, double* out) {
+  __shared__ double red[256];
+  double acc = 0.0;
+  for (int b = threadIdx.x; b < nparts; b += blockDim.x) acc = __dadd_rn(acc, part[b]);
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if (threadIdx.x < w) red[threadIdx.x] = __dadd_rn(red[threadIdx.x], red[threadIdx.x + w]);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *out = __dmul_rn(0.5, red[0]);
 }
 
 template <typename T>
@@ -830,19 +876,7 @@ __global__ void __launch_bounds__(256) fit_special_post(FitGrid<T> g, SpecialEdg
     T* U = comp_ptr(g.Ux, g.Uy, g.Uz, sp.comp[e]);
     U[sp.slot[e]] = sp.out[e];
   }
-  if (blockIdx.x == 0) {
-    // fixed-order reduction of the per-block flux partials
-    __shared__ double red[256];
-    double acc = 0.0;
-    for (int b = threadIdx.x; b < nparts; b += blockDim.x) acc = __dadd_rn(acc, sp.flux_part[b]);
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w) red[threadIdx.x] = __dadd_rn(red[threadIdx.x], red[threadIdx.x + w]);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) flux[*step_counter] = __dmul_rn(0.5, red[0]);
-  }
+  if (blockIdx.x == 0) flux_total(sp.flux_part, nparts, flux + *step_counter);
 }
 
 template <typename T>
@@ -1048,11 +1082,17 @@ __global__ void __launch_bounds__(256) fit_class_insert(FitGrid<T> g, FitClassWo
   });
 }
 
+__global__ void fit_class_special(FitClassSlots c, const int8_t* comp, const int64_t* slot, int n);
+
 // One thread per table slot: number the occupied slots and fill the tables.
 template <typename T>
 __global__ void __launch_bounds__(256) fit_class_number(FitGrid<T> g, FitClassWork w, int kind) {
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= kClassTable) return;
+  if (h == 0) {  // slots without an updated dof: the H half puts the face's own value back
+    (kind == 0 ? g.lut_e : g.lut_f)[2 * kNoClass] = (T)-0.0;
+    (kind == 0 ? g.lut_e : g.lut_f)[2 * kNoClass + 1] = (T)0;
+  }
   const unsigned long long key = w.keys[kind][h];
   if (key == kNoKey) return;
   const int id = atomicAdd(&w.count[kind], 1);
@@ -1089,7 +1129,8 @@ __global__ void __launch_bounds__(256) fit_class_assign(FitGrid<T> g, FitClassWo
 }
 
 template <typename T>
-cudaError_t fit_build_classes(const FitGrid<T>& g, const FitClassWork& w, int ncls[2], cudaStream_t st) {
+cudaError_t fit_build_classes(const FitGrid<T>& g, const SpecialEdges<T>& sp, const FitClassWork& w, int ncls[2],
+                              cudaStream_t st) {
   for (int q = 0; q < 2; q++)
     if (cudaMemsetAsync(w.keys[q], 0xff, sizeof(unsigned long long) * kClassTable, st) != cudaSuccess)
       return cudaGetLastError();
@@ -1105,32 +1146,25 @@ cudaError_t fit_build_classes(const FitGrid<T>& g, const FitClassWork& w, int nc
   for (int q = 0; q < 2; q++) ncls[q] = (c[2] || c[q] > kMaxClasses) ? -1 : c[q];
   if (ncls[0] < 0 || ncls[1] < 0) return cudaSuccess;
   fit_class_assign<T><<<grd, blk, 0, st>>>(g, w);
+  if (sp.n > 0) {
+    FitClassSlots c;
+    for (int a = 0; a < 3; a++) c.Ke[a] = g.Ke[a];
+    fit_class_special<<<(sp.n + 255) / 256, 256, 0, st>>>(c, sp.comp, sp.slot, sp.n);
+  }
   return cudaGetLastError();
 }
-template cudaError_t fit_build_classes<double>(const FitGrid<double>&, const FitClassWork&, int*, cudaStream_t);
-template cudaError_t fit_build_classes<float>(const FitGrid<float>&, const FitClassWork&, int*, cudaStream_t);
+template cudaError_t fit_build_classes<double>(const FitGrid<double>&, const SpecialEdges<double>&, const FitClassWork&, int*,
+                                                 cudaStream_t);
+template cudaError_t fit_build_classes<float>(const FitGrid<float>&, const SpecialEdges<float>&, const FitClassWork&, int*,
+                                                cudaStream_t);
 
 // Plane-per-block E and H updates with the coefficients streamed per dof
-// (CLS false: M_h, M_q / M_nu, M_mu arrays) or looked up by class (CLS true:
-// a 2-byte class per dof into the class tables); same arithmetic as
-// fit_e_kernel / fit_h_kernel.  Every load of a node comes first and the
-// stores last: the six arrays do not alias, which the compiler cannot know,
-// and with stores in between it would wait for each dof's loads in turn.
-template <typename T, bool CLS>
-__device__ __forceinline__ void coef_pair(const T* const* C0, const T* const* C1, const uint16_t* const* K,
-                                          const T* lut, int a, int64_t s, T& c0, T& c1) {
-  if (CLS) {
-    const int c = __ldg(K[a] + s);
-    c0 = __ldg(lut + 2 * c);
-    c1 = __ldg(lut + 2 * c + 1);
-  } else {
-    c0 = __ldg(C0[a] + s);
-    c1 = __ldg(C1[a] + s);
-  }
-}
-
-template <typename T, bool CLS>
-__device__ __forceinline__ void e_update_streamed(const FitGrid<T>& g) {
+// (M_h, M_q / M_nu, M_mu arrays); same arithmetic as fit_e_kernel /
+// fit_h_kernel.  Every load of a node comes first and the stores last: the six
+// arrays do not alias, which the compiler cannot know, and with stores in
+// between it would wait for each dof's loads in turn.
+template <typename T>
+__global__ void __launch_bounds__(256) fit_e_coef(FitGrid<T> g) {
   using A = Ar<T>;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1149,19 +1183,22 @@ __device__ __forceinline__ void e_update_streamed(const FitGrid<T>& g) {
     fy_b = g.Fy[s - g.sxy];
     fz_y = g.Fz[s - g.sx];
     ux = g.Ux[s];
-    coef_pair<T, CLS>(g.Ch, g.Cq, g.Ke, g.lut_e, 0, s, h0, q0);
+    h0 = __ldg(g.Ch[0] + s);
+    q0 = __ldg(g.Cq[0] + s);
   }
   if (ey) {
     fx_b = g.Fx[s - g.sxy];
     fz_x = g.Fz[s - 1];
     uy = g.Uy[s];
-    coef_pair<T, CLS>(g.Ch, g.Cq, g.Ke, g.lut_e, 1, s, h1, q1);
+    h1 = __ldg(g.Ch[1] + s);
+    q1 = __ldg(g.Cq[1] + s);
   }
   if (ez) {
     fx_y = g.Fx[s - g.sx];
     fy_x = g.Fy[s - 1];
     uz = g.Uz[s];
-    coef_pair<T, CLS>(g.Ch, g.Cq, g.Ke, g.lut_e, 2, s, h2, q2);
+    h2 = __ldg(g.Ch[2] + s);
+    q2 = __ldg(g.Cq[2] + s);
   }
   if (ex) {
     const T cf = A::sub(A::add(A::sub(fy_b, fz_y), fz), fy);
@@ -1177,9 +1214,14 @@ __device__ __forceinline__ void e_update_streamed(const FitGrid<T>& g) {
   }
 }
 
-// A skipped face (M_nu = -0.0) gets its own value back.
-template <typename T, bool CLS>
-__device__ __forceinline__ void h_update_streamed(const FitGrid<T>& g, int* step_counter) {
+// A face the H update skips has M_nu = -0.0: it gets its own value back.
+template <typename T>
+__device__ __forceinline__ bool face_skipped(T mnu) {
+  return mnu == (T)0 && signbit(mnu);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) fit_h_coef(FitGrid<T> g, int* step_counter) {
   using A = Ar<T>;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1199,46 +1241,375 @@ __device__ __forceinline__ void h_update_streamed(const FitGrid<T>& g, int* step
     uz_y = g.Uz[s + g.sx];
     uy_z = g.Uy[s + g.sxy];
     fx = g.Fx[s];
-    coef_pair<T, CLS>(g.Cn, g.Cm, g.Kf, g.lut_f, 0, s, n0, m0);
+    n0 = __ldg(g.Cn[0] + s);
+    m0 = __ldg(g.Cm[0] + s);
   }
   if (hy) {
     uz_x = g.Uz[s + 1];
     ux_z = g.Ux[s + g.sxy];
     fy = g.Fy[s];
-    coef_pair<T, CLS>(g.Cn, g.Cm, g.Kf, g.lut_f, 1, s, n1, m1);
+    n1 = __ldg(g.Cn[1] + s);
+    m1 = __ldg(g.Cm[1] + s);
   }
   if (hz) {
     uy_x = g.Uy[s + 1];
     ux_y = g.Ux[s + g.sx];
     fz = g.Fz[s];
-    coef_pair<T, CLS>(g.Cn, g.Cm, g.Kf, g.lut_f, 2, s, n2, m2);
+    n2 = __ldg(g.Cn[2] + s);
+    m2 = __ldg(g.Cm[2] + s);
   }
-  auto skip = [](T v) { return v == (T)0 && signbit(v); };
   if (hx) {
     const T cs = A::sub(A::add(A::sub(uy, uz), uz_y), uy_z);
-    g.Fx[s] = skip(n0) ? fx : A::mul(n0, face_flux(m0, fx, dt, cs));
+    g.Fx[s] = face_skipped(n0) ? fx : A::mul(n0, face_flux(m0, fx, dt, cs));
   }
   if (hy) {
     const T cs = A::sub(A::add(A::sub(ux, uz), uz_x), ux_z);
-    g.Fy[s] = skip(n1) ? fy : A::mul(n1, face_flux(m1, fy, -dt, cs));
+    g.Fy[s] = face_skipped(n1) ? fy : A::mul(n1, face_flux(m1, fy, -dt, cs));
   }
   if (hz) {
     const T cs = A::sub(A::add(A::sub(ux, uy), uy_x), ux_y);
-    g.Fz[s] = skip(n2) ? fz : A::mul(n2, face_flux(m2, fz, dt, cs));
+    g.Fz[s] = face_skipped(n2) ? fz : A::mul(n2, face_flux(m2, fz, dt, cs));
   }
 }
 
+// ------------------------------------------------------- coefficient classes
+// The class variant makes a leapfrog step of two launches.  fit_e_class: the
+// special edges' blocks first (their source chain is the longest), blocks
+// that set the probes' face values aside, then the interior edges.
+// fit_h_class: the probes' blocks, the boundary flux sum, then the faces.
+// Nothing in a launch reads what the launch writes: the E half reads F and
+// each edge's own U, the H half reads U and each face's own F, an edge has one
+// writer (the special edges carry kNoClass, which the interior part leaves
+// alone), and the probes read the faces' old values from the copy.
+//
+// Bounds: launch latency on small grids, DRAM on large ones (256^3 FP32: the
+// E half moves 0.66 GB, the H half 0.66 GB; 135 and 121 us, 0.75 and 0.84 of
+// the measured copy bandwidth; one slot per thread in five launches took 158
+// and 162 us, a 24^3 FP64 step 64 us against 6).  Three blocks of 256 an SM
+// leave room for every load of a thread in flight at once (80 registers);
+// four (64 registers) spill and ran 20 % slower at 256^3.
+//
+// Interior part: a thread takes 16 bytes of consecutive slots of the linear
+// arrays (four FP32 or two FP64), with aligned 16-byte loads for the slots and
+// their y and z neighbours and a lane shuffle for the x neighbour.  There are
+// no position tests: slots that hold no updated dof carry kNoClass, and the
+// arrays are padded by a plane on both sides so that every neighbour can be
+// read.  Same arithmetic as fit_e_kernel / fit_h_kernel.
 template <typename T>
-__global__ void __launch_bounds__(256) fit_e_coef(FitGrid<T> g) { e_update_streamed<T, false>(g); }
+struct Pack;
+template <>
+struct Pack<float> {
+  static constexpr int N = 4;
+  float v[4];
+  __device__ __forceinline__ void load(const float* p) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  }
+  __device__ __forceinline__ void store(float* p) const {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+};
+template <>
+struct Pack<double> {
+  static constexpr int N = 2;
+  double v[2];
+  __device__ __forceinline__ void load(const double* p) {
+    const double2 q = *reinterpret_cast<const double2*>(p);
+    v[0] = q.x; v[1] = q.y;
+  }
+  __device__ __forceinline__ void store(double* p) const { *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]); }
+};
+__device__ __forceinline__ void load_classes(uint16_t* c, const uint16_t* p, float) {
+  const ushort4 q = __ldg(reinterpret_cast<const ushort4*>(p));
+  c[0] = q.x; c[1] = q.y; c[2] = q.z; c[3] = q.w;
+}
+__device__ __forceinline__ void load_classes(uint16_t* c, const uint16_t* p, double) {
+  const ushort2 q = __ldg(reinterpret_cast<const ushort2*>(p));
+  c[0] = q.x; c[1] = q.y;
+}
+__device__ __forceinline__ void load_pair(const float* lut, int c, float& a, float& b) {
+  const float2 q = __ldg(reinterpret_cast<const float2*>(lut) + c);
+  a = q.x; b = q.y;
+}
+__device__ __forceinline__ void load_pair(const double* lut, int c, double& a, double& b) {
+  const double2 q = __ldg(reinterpret_cast<const double2*>(lut) + c);
+  a = q.x; b = q.y;
+}
+
+// the pack one slot to the left / right: the neighbour lanes' border values,
+// the warp's own border from memory
 template <typename T>
-__global__ void __launch_bounds__(256) fit_h_coef(FitGrid<T> g, int* step_counter) {
-  h_update_streamed<T, false>(g, step_counter);
+__device__ __forceinline__ Pack<T> shift_left(const Pack<T>& a, const T* p, bool ok) {
+  Pack<T> r;
+  T e = __shfl_up_sync(0xffffffffu, a.v[Pack<T>::N - 1], 1);
+  if ((threadIdx.x & 31) == 0 && ok) e = p[-1];
+  r.v[0] = e;
+#pragma unroll
+  for (int q = 1; q < Pack<T>::N; q++) r.v[q] = a.v[q - 1];
+  return r;
 }
 template <typename T>
-__global__ void __launch_bounds__(256) fit_e_class(FitGrid<T> g) { e_update_streamed<T, true>(g); }
+__device__ __forceinline__ Pack<T> shift_right(const Pack<T>& a, const T* p, bool ok, bool last) {
+  Pack<T> r;
+  T e = __shfl_down_sync(0xffffffffu, a.v[0], 1);
+  if (ok && ((threadIdx.x & 31) == 31 || last)) e = p[Pack<T>::N];
+#pragma unroll
+  for (int q = 0; q + 1 < Pack<T>::N; q++) r.v[q] = a.v[q + 1];
+  r.v[Pack<T>::N - 1] = e;
+  return r;
+}
+
+// the coefficient pairs of a pack's slots
 template <typename T>
-__global__ void __launch_bounds__(256) fit_h_class(FitGrid<T> g, int* step_counter) {
-  h_update_streamed<T, true>(g, step_counter);
+struct Coef {
+  uint16_t c[Pack<T>::N];
+  Pack<T> a, b;
+  __device__ __forceinline__ void classes(const uint16_t* K) { load_classes(c, K, T()); }
+  __device__ __forceinline__ void pairs(const T* lut) {
+#pragma unroll
+    for (int q = 0; q < Pack<T>::N; q++) load_pair(lut, c[q], a.v[q], b.v[q]);
+  }
+};
+
+template <typename T>
+__device__ __forceinline__ void store_edges(T* U, const Coef<T>& k, const Pack<T>& u, const Pack<T>& cf, T dt) {
+  using A = Ar<T>;
+  Pack<T> r;
+  bool all = true;
+#pragma unroll
+  for (int q = 0; q < Pack<T>::N; q++) {
+    r.v[q] = A::mul(k.a.v[q], A::add(A::mul(k.b.v[q], u.v[q]), A::mul(dt, cf.v[q])));
+    all = all && k.c[q] != kNoClass;
+  }
+  if (all) {
+    r.store(U);
+  } else {
+#pragma unroll
+    for (int q = 0; q < Pack<T>::N; q++)
+      if (k.c[q] != kNoClass) U[q] = r.v[q];
+  }
+}
+
+template <typename T, bool kPdl>
+__device__ __forceinline__ void e_interior(const FitGrid<T>& g, int64_t s) {
+  using A = Ar<T>;
+  constexpr int N = Pack<T>::N;
+  const bool ok = s < g.nslot;
+  Pack<T> fx, fy, fz, fxy, fxz, fyz, fzy, ux, uy, uz;
+  Coef<T> kx, ky, kz;
+  if (kPdl && ok) {
+    kx.classes(g.Ke[0] + s);
+    ky.classes(g.Ke[1] + s);
+    kz.classes(g.Ke[2] + s);
+  }
+  if (kPdl) cudaGridDependencySynchronize();
+  if (ok) {
+    fx.load(g.Fx + s);
+    fy.load(g.Fy + s);
+    fz.load(g.Fz + s);
+    fxy.load(g.Fx + s - g.sx);
+    fxz.load(g.Fx + s - g.sxy);
+    fyz.load(g.Fy + s - g.sxy);
+    fzy.load(g.Fz + s - g.sx);
+    ux.load(g.Ux + s);
+    uy.load(g.Uy + s);
+    uz.load(g.Uz + s);
+    if (!kPdl) {
+      kx.classes(g.Ke[0] + s);
+      ky.classes(g.Ke[1] + s);
+      kz.classes(g.Ke[2] + s);
+    }
+    kx.pairs(g.lut_e);
+    ky.pairs(g.lut_e);
+    kz.pairs(g.lut_e);
+  }
+  const Pack<T> fyx = shift_left(fy, g.Fy + s, ok), fzx = shift_left(fz, g.Fz + s, ok);
+  if (!ok) return;
+  const T dt = (T)g.dt;
+  Pack<T> cx, cy, cz;
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    cx.v[q] = A::sub(A::add(A::sub(fyz.v[q], fzy.v[q]), fz.v[q]), fy.v[q]);
+    cy.v[q] = -A::sub(A::add(A::sub(fxz.v[q], fzx.v[q]), fz.v[q]), fx.v[q]);
+    cz.v[q] = A::sub(A::add(A::sub(fxy.v[q], fyx.v[q]), fy.v[q]), fx.v[q]);
+  }
+  store_edges(g.Ux + s, kx, ux, cx, dt);
+  store_edges(g.Uy + s, ky, uy, cy, dt);
+  store_edges(g.Uz + s, kz, uz, cz, dt);
+}
+
+template <typename T>
+__device__ __forceinline__ void store_faces(T* F, const Coef<T>& k, const Pack<T>& f, const Pack<T>& cs, T dt) {
+  Pack<T> r;
+#pragma unroll
+  for (int q = 0; q < Pack<T>::N; q++)
+    r.v[q] = face_skipped(k.a.v[q]) ? f.v[q] : Ar<T>::mul(k.a.v[q], face_flux(k.b.v[q], f.v[q], dt, cs.v[q]));
+  r.store(F);
+}
+
+template <typename T, bool kPdl>
+__device__ __forceinline__ void h_interior(const FitGrid<T>& g, int64_t s) {
+  using A = Ar<T>;
+  constexpr int N = Pack<T>::N;
+  const bool ok = s < g.nslot;
+  Pack<T> ux, uy, uz, uxy, uxz, uyz, uzy, fx, fy, fz;
+  Coef<T> kx, ky, kz;
+  if (kPdl && ok) {
+    kx.classes(g.Kf[0] + s);
+    ky.classes(g.Kf[1] + s);
+    kz.classes(g.Kf[2] + s);
+  }
+  if (kPdl) cudaGridDependencySynchronize();
+  if (ok) {
+    ux.load(g.Ux + s);
+    uy.load(g.Uy + s);
+    uz.load(g.Uz + s);
+    uxy.load(g.Ux + s + g.sx);
+    uxz.load(g.Ux + s + g.sxy);
+    uyz.load(g.Uy + s + g.sxy);
+    uzy.load(g.Uz + s + g.sx);
+    fx.load(g.Fx + s);
+    fy.load(g.Fy + s);
+    fz.load(g.Fz + s);
+    if (!kPdl) {
+      kx.classes(g.Kf[0] + s);
+      ky.classes(g.Kf[1] + s);
+      kz.classes(g.Kf[2] + s);
+    }
+    kx.pairs(g.lut_f);
+    ky.pairs(g.lut_f);
+    kz.pairs(g.lut_f);
+  }
+  const bool last = s + N >= g.nslot;
+  const Pack<T> uyx = shift_right(uy, g.Uy + s, ok, last), uzx = shift_right(uz, g.Uz + s, ok, last);
+  if (!ok) return;
+  const T dt = (T)g.dt;
+  Pack<T> cx, cy, cz;
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    cx.v[q] = A::sub(A::add(A::sub(uy.v[q], uz.v[q]), uzy.v[q]), uyz.v[q]);
+    cy.v[q] = A::sub(A::add(A::sub(ux.v[q], uz.v[q]), uzx.v[q]), uxz.v[q]);
+    cz.v[q] = A::sub(A::add(A::sub(ux.v[q], uy.v[q]), uyx.v[q]), uxy.v[q]);
+  }
+  store_faces(g.Fx + s, kx, fx, cx, dt);
+  store_faces(g.Fy + s, ky, fy, cy, -dt);
+  store_faces(g.Fz + s, kz, fz, cz, dt);
+}
+
+// The two faces of probe p's cell across axis a, low and high.
+__device__ __forceinline__ int64_t probe_slot(const ProbeSet& pr, int p, int64_t sx, int64_t sxy) {
+  return (int64_t)pr.ci[p] + sx * pr.cj[p] + sxy * pr.ck[p];
+}
+
+// Both kernels let the next launch's blocks become resident at once and read
+// the static tables (classes, coefficients, source tables) before they wait
+// for the launch before them.
+//
+// A launch's blocks: `extra` blocks of other work spread evenly among the
+// interior's, so that on a large grid their long load chains run beside the
+// interior's streams (all of them first, the 514 source-wall blocks of a 256^3
+// grid filled most of the first wave).  Returns the extra block's number, or
+// -1 with the interior block's in b.
+__device__ __forceinline__ int extra_block(int extra, int& b) {
+  const int every = extra > 0 ? (int)gridDim.x / extra : 1;
+  const int x = b / every;
+  if (x < extra && b % every == 0) return x;
+  b -= x < extra ? x + 1 : extra;
+  return -1;
+}
+
+// step_counter[0] is the step being made; the E half copies it to
+// step_counter[1], from where the H half reads it and advances [0].
+template <typename T, bool kPdl>
+__global__ void __launch_bounds__(256, 3) fit_e_class(FitGrid<T> g, SpecialEdges<T> sp, ProbeSet pr, int* step_counter,
+                                                   int nsb, int npb) {
+  if (kPdl) cudaTriggerProgrammaticLaunchCompletion();
+  int b = blockIdx.x;
+  const int x = extra_block(nsb + npb + 1, b) - 1;
+  if (x == -1) {
+    if (kPdl) cudaGridDependencySynchronize();
+    if (threadIdx.x == 0) step_counter[1] = step_counter[0];
+    return;
+  }
+  if (x >= 0 && x < nsb) {
+    special_edges<T, true, kPdl>(g, sp, step_counter, x);
+    return;
+  }
+  if (x >= nsb) {
+    const int t = (x - nsb) * 256 + threadIdx.x;
+    const int p = t / 6, q = t % 6, a = q >> 1;
+    int64_t s = 0;
+    if (p < pr.n) s = probe_slot(pr, p, g.sx, g.sxy) + ((q & 1) ? (a == 0 ? 1 : (a == 1 ? g.sx : g.sxy)) : 0);
+    if (kPdl) cudaGridDependencySynchronize();
+    if (p >= pr.n || pr.slot_of_step[*step_counter] < 0) return;
+    ((T*)pr.faces)[t] = comp_ptr(g.Fx, g.Fy, g.Fz, a)[s];
+    return;
+  }
+  e_interior<T, kPdl>(g, ((int64_t)b * 256 + threadIdx.x) * Pack<T>::N);
+}
+
+template <typename T, bool kPdl>
+__global__ void __launch_bounds__(256, 3) fit_h_class(FitGrid<T> g, ProbeSet pr, int* step_counter, double* flux,
+                                                   const double* flux_part, int nparts, int npb) {
+  if (kPdl) cudaTriggerProgrammaticLaunchCompletion();
+  int b = blockIdx.x;
+  const int x = extra_block(npb + 1, b);
+  if (x > 0) {  // one thread per probe and field component
+    const int t = (x - 1) * 256 + threadIdx.x;
+    const int p = t / 6, c = t % 6, a = c % 3;
+    const int64_t da = a == 0 ? 1 : (a == 1 ? g.sx : g.sxy);
+    int64_t s = 0;
+    T mnu[2] = {0, 0}, mmu[2] = {0, 0};
+    double inv_mu = 0.0;
+    if (p < pr.n) {
+      s = probe_slot(pr, p, g.sx, g.sxy);
+      inv_mu = pr.inv_mu[3 * p + a];
+#pragma unroll
+      for (int q = 0; q < 2; q++) load_pair(g.lut_f, g.Kf[a][s + q * da], mnu[q], mmu[q]);
+    }
+    if (kPdl) cudaGridDependencySynchronize();
+    if (p >= pr.n) return;
+    const int slotn = pr.slot_of_step[step_counter[1]];
+    if (slotn < 0) return;
+    const double vol = __dmul_rn(__dmul_rn(g.len[0], g.len[1]), g.len[2]);
+    double* out = pr.samples + (int64_t)slotn * pr.n * 6 + t;
+    if (c < 3) {
+      const T* U = comp_ptr(g.Ux, g.Uy, g.Uz, a);
+      const int64_t d0 = a == 0 ? g.sx : 1, d1 = a == 2 ? g.sx : g.sxy;
+      const double w = (a == 0 ? __dmul_rn(g.len[1], g.len[2])
+                               : (a == 1 ? __dmul_rn(g.len[0], g.len[2]) : __dmul_rn(g.len[0], g.len[1]))) / 4;
+      const double v0 = (double)U[s], v1 = (double)U[s + d0], v2 = (double)U[s + d1], v3 = (double)U[s + d0 + d1];
+      *out = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(v0, w), __dmul_rn(v1, w)), __dmul_rn(v2, w)),
+                       __dmul_rn(v3, w)) / vol;
+      return;
+    }
+    const T dt = (T)g.dt;
+    const double half = __dmul_rn(0.5, a == 0 ? g.len[0] : (a == 1 ? g.len[1] : g.len[2]));
+    T B[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int64_t f = s + q * da;
+      const T cs = a == 0 ? curl_x(g, f) : (a == 1 ? curl_y(g, f) : curl_z(g, f));
+      B[q] = face_flux(mmu[q], ((const T*)pr.faces)[6 * p + 2 * a + q], a == 1 ? -dt : dt, cs);
+      if (face_skipped(mnu[q])) B[q] = (T)0;
+    }
+    const double h = __dadd_rn(__dmul_rn((double)B[0], half), __dmul_rn((double)B[1], half));
+    *out = __dmul_rn(inv_mu, h) / vol;
+    return;
+  }
+  if (x == 0) {
+    if (kPdl) cudaGridDependencySynchronize();
+    flux_total(flux_part, nparts, flux + step_counter[1]);
+    if (threadIdx.x == 0) step_counter[0] = step_counter[1] + 1;
+    return;
+  }
+  h_interior<T, kPdl>(g, ((int64_t)b * 256 + threadIdx.x) * Pack<T>::N);
+}
+
+// Marks the special edges' slots as not updated by the interior part.
+__global__ void fit_class_special(FitClassSlots c, const int8_t* comp, const int64_t* slot, int n) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < n) c.Ke[comp[e]][slot[e]] = kNoClass;
 }
 
 // Joule loss partials: one thread per node slot sums Si_e (U_old + U)_e^2 over
@@ -1305,19 +1676,26 @@ __global__ void __launch_bounds__(256) fit_loss_finish(const double* part, int n
 }
 
 // ---------------------------------------------------------------- launchers
-// Block shape of the streamed variants (x by y node slots of one plane; at
-// most 256 threads, the kernels' launch bound).  32 x 4 and 64 x 2 measured
-// fastest at 256^3 and 512^3 (FP32, B200): 4 % below 32 x 8; 32 x 1 took twice
-// as long, 256 x 1 and 16 x 16 were slower than 32 x 8.
+// Block shape of the coefficient-array variant (x by y node slots of one
+// plane; at most 256 threads, the kernels' launch bound).  32 x 4 and 64 x 2
+// measured fastest at 256^3 and 512^3 (FP32, B200): 4 % below 32 x 8; 32 x 1
+// took twice as long, 256 x 1 and 16 x 16 were slower than 32 x 8.
 #ifndef TF_FIT_SBX
 #define TF_FIT_SBX 32
 #endif
 #ifndef TF_FIT_SBY
 #define TF_FIT_SBY 4
 #endif
+// Programmatic dependent launch of the class kernels, for launches of up to
+// this many blocks.  It hides the launch gap and the tables' load latency
+// (step at 24^3 FP64 7.7 -> 6.1 us, 64^3 FP32 8.9 -> 7.0, 80^3 FP64, 1,130
+// blocks, 15.0 -> 14.2); on large grids the wait keeps a thread's table loads
+// apart from its field loads, which costs more (256^3 FP32 250 -> 260 us).
+constexpr unsigned kPdlBlocks = 2048;
 // Kernel variants for the E and H halves (all compute bit-identical results):
 // 0 one thread per node slot, 1 z-march over 4 planes, 2 z-march over 16,
-// 3 one thread per node slot with per-dof coefficient arrays.
+// 3 one thread per node slot with per-dof coefficient arrays, 4 z-march with
+// TMA-staged planes, 5 coefficient classes (both halves together).
 template <typename T>
 void fit_launch_step(const FitGrid<T>& g, const SpecialEdges<T>& sp, const ProbeSet& pr, int* step_counter,
                      double* flux, cudaStream_t st, cudaEvent_t* ev, int e_variant, int h_variant,
@@ -1326,7 +1704,7 @@ void fit_launch_step(const FitGrid<T>& g, const SpecialEdges<T>& sp, const Probe
   // loss (optional): Joule loss of the E half step
   dim3 blk(32, 8, 1);
   dim3 grd((unsigned)((g.Nx + 1 + 31) / 32), (unsigned)((g.Ny + 1 + 7) / 8), (unsigned)(g.Nz + 1));
-  // the streamed variants (3, 5): one node slot per thread, one plane per block
+  // the coefficient-array variant (3): one node slot per thread, one plane per block
   const dim3 sblk(TF_FIT_SBX, TF_FIT_SBY, 1);
   const dim3 sgrd((unsigned)((g.Nx + TF_FIT_SBX) / TF_FIT_SBX), (unsigned)((g.Ny + TF_FIT_SBY) / TF_FIT_SBY),
                   (unsigned)(g.Nz + 1));
@@ -1334,6 +1712,7 @@ void fit_launch_step(const FitGrid<T>& g, const SpecialEdges<T>& sp, const Probe
     return dim3((unsigned)((g.Nx + 1 + 31) / 32), (unsigned)((g.Ny + 1 + 7) / 8), (unsigned)((g.Nz + 1 + kc - 1) / kc));
   };
   const int nsb = (sp.n + 255) / 256;
+  const bool cls = e_variant == 5 && h_variant == 5 && g.lut_e;
   if (ev) cudaEventRecord(ev[0], st);
   if (loss) {
     const size_t bytes = (size_t)(g.sxy * (g.Nz + 1)) * sizeof(T);
@@ -1341,11 +1720,38 @@ void fit_launch_step(const FitGrid<T>& g, const SpecialEdges<T>& sp, const Probe
     cudaMemcpyAsync(loss->Oy, g.Uy, bytes, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(loss->Oz, g.Uz, bytes, cudaMemcpyDeviceToDevice, st);
   }
+  if (cls) {
+    const unsigned nib = (unsigned)((g.nslot / Pack<T>::N + 255) / 256);
+    const int npb = (6 * pr.n + 255) / 256;
+    if (ev) cudaEventRecord(ev[1], st);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    const bool pdl = nsb + npb + 1 + nib <= kPdlBlocks;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.gridDim = dim3(nsb + npb + 1 + nib);
+    cudaLaunchKernelEx(&cfg, pdl ? fit_e_class<T, true> : fit_e_class<T, false>, g, sp, pr, step_counter, nsb, npb);
+    if (ev) cudaEventRecord(ev[2], st);
+    if (loss) {
+      fit_loss_kernel<T><<<grd, blk, 0, st>>>(g, *loss);
+      fit_loss_finish<<<1, 256, 0, st>>>(loss->part, loss->nparts, loss->loss, step_counter);
+    }
+    if (ev) cudaEventRecord(ev[3], st);
+    if (ev) cudaEventRecord(ev[4], st);
+    cfg.gridDim = dim3(npb + 1 + nib);
+    cudaLaunchKernelEx(&cfg, pdl ? fit_h_class<T, true> : fit_h_class<T, false>, g, pr, step_counter, flux,
+                       (const double*)sp.flux_part, nsb, npb);
+    if (ev) cudaEventRecord(ev[5], st);
+    return;
+  }
   if (sp.n > 0) fit_special_pre<T><<<nsb, 256, 0, st>>>(g, sp, step_counter);
   if (ev) cudaEventRecord(ev[1], st);
   if (e_variant == 0) fit_e_kernel<T><<<grd, blk, 0, st>>>(g);
   else if (e_variant == 3) fit_e_coef<T><<<sgrd, sblk, 0, st>>>(g);
-  else if (e_variant == 5 && g.lut_e) fit_e_class<T><<<sgrd, sblk, 0, st>>>(g);
   else if (e_variant == 4 && tma)
     fit_e_tma<T><<<mgrid(16), dim3(kTmaTX, kTmaTY + 1), 0, st>>>(g, 16, tma->F[0], tma->F[1], tma->F[2], tma->U[0], tma->U[1], tma->U[2],
                                              tma->err);
@@ -1364,7 +1770,6 @@ void fit_launch_step(const FitGrid<T>& g, const SpecialEdges<T>& sp, const Probe
   if (ev) cudaEventRecord(ev[4], st);
   if (h_variant == 0) fit_h_kernel<T><<<grd, blk, 0, st>>>(g, step_counter);
   else if (h_variant == 3) fit_h_coef<T><<<sgrd, sblk, 0, st>>>(g, step_counter);
-  else if (h_variant == 5 && g.lut_f) fit_h_class<T><<<sgrd, sblk, 0, st>>>(g, step_counter);
   else if (h_variant == 4 && tma)
     fit_h_tma<T><<<mgrid(16), dim3(kTmaTX, kTmaTY + 1), 0, st>>>(g, 16, step_counter, tma->U[0], tma->U[1], tma->U[2], tma->F[0],
                                              tma->F[1], tma->F[2], tma->err);
@@ -1375,7 +1780,8 @@ void fit_launch_step(const FitGrid<T>& g, const SpecialEdges<T>& sp, const Probe
   if (ev) cudaEventRecord(ev[5], st);
 }
 
-int fit_kernels_per_step(int n_special, int n_probes, bool losses) {
+int fit_kernels_per_step(int n_special, int n_probes, bool losses, bool classes) {
+  if (classes) return 2 + (losses ? 2 : 0);
   return 3 + (n_special > 0) + (n_probes > 0) + (losses ? 2 : 0);
 }
 

@@ -28,6 +28,7 @@ struct FitGrid {
   const uint8_t* mat;  // [Nz][Ny][Nx] compact material index per cell
   int Nx, Ny, Nz;
   int64_t sx, sxy;     // strides of the state arrays
+  int64_t nslot;       // sxy (Nz + 1); each state array has a zeroed plane and a row more on both sides
   double dt;
   // per-material tables, 3 entries per material (axis x,y,z)
   const double* P;     // da_a * eps_aa           (edge permittivity share)
@@ -44,12 +45,13 @@ struct FitGrid {
   // computed once from the tables above by fit_coef_kernel: M_h, M_q per
   // edge, M_nu, M_mu per face (M_nu = -0.0 marks a face the H update skips)
   T *Ch[3], *Cq[3], *Cn[3], *Cm[3];
-  // optional coefficient classes: a uint16 class per updated edge and face
-  // (state-array shape, one array per axis) into tables of coefficient
-  // pairs, lut_e[2c] = M_h, lut_e[2c+1] = M_q and lut_f[2c] = M_nu,
-  // lut_f[2c+1] = M_mu (M_nu = -0.0 marks a face the H update skips).  A
-  // class is a distinct tuple (axis, materials of the dof's cells), and its
-  // pair is computed from the tuple by the same functions as above.
+  // coefficient classes: a uint16 class per updated edge and face
+  // (state-array shape, one array per axis; kNoClass on every other slot and
+  // on the special edges) into tables of coefficient pairs, lut_e[2c] = M_h,
+  // lut_e[2c+1] = M_q and lut_f[2c] = M_nu, lut_f[2c+1] = M_mu (M_nu = -0.0
+  // marks a face the H update skips).  A class is a distinct tuple (axis,
+  // materials of the dof's cells), and its pair is computed from the tuple
+  // by the same functions as above.
   uint16_t *Ke[3], *Kf[3];
   T *lut_e, *lut_f;
 };
@@ -57,6 +59,10 @@ struct FitGrid {
 // Hash tables of the class build (device memory, kClassTable slots each).
 constexpr int kClassTable = 1 << 20;
 constexpr int kMaxClasses = 65535;
+constexpr uint16_t kNoClass = 65535;  // the tables have kMaxClasses + 1 pairs
+struct FitClassSlots {
+  uint16_t* Ke[3];
+};
 struct FitClassWork {
   unsigned long long* keys[2];  // edge and face tuples, ~0 empty
   int* ids[2];                  // dense class of an occupied slot
@@ -114,10 +120,6 @@ struct FitTmaMaps {
 
 template <typename T>
 cudaError_t fit_build_coefficients(const FitGrid<T>& g, cudaStream_t st);
-// Fills g.Ke, g.Kf and the class tables; ncls[0..1] receive the edge and
-// face class counts, -1 when there are more than kMaxClasses.
-template <typename T>
-cudaError_t fit_build_classes(const FitGrid<T>& g, const FitClassWork& w, int ncls[2], cudaStream_t st);
 
 struct ProbeSet {
   int n;
@@ -125,6 +127,13 @@ struct ProbeSet {
   const double* inv_mu;                          // [n][3] 1/mu_aa of the cell material
   double* samples;                               // [slots][n][6]
   const int* slot_of_step;                       // print slot per step, -1 none
+  void* faces;                                   // [n][3 axes][2] T: the cells' face values before the H half
 };
+
+// Fills g.Ke, g.Kf and the class tables; ncls[0..1] receive the edge and
+// face class counts, -1 when there are more than kMaxClasses.
+template <typename T>
+cudaError_t fit_build_classes(const FitGrid<T>& g, const SpecialEdges<T>& sp, const FitClassWork& w, int ncls[2],
+                              cudaStream_t st);
 
 }  // namespace tf
