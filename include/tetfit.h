@@ -84,7 +84,9 @@ typedef struct tf_info {
   uint64_t n_free, nnz_system;         /* gfdtd: CG unknowns and nonzeros of A    */
   uint64_t nnz_operators;              /* nonzeros of H (dga) or of E (gfdtd)     */
   uint32_t cg_blocks;                  /* gfdtd: blocks of the persistent CG kernel */
-  int32_t cg_variant;                  /* gfdtd: CG variant the autotuner picked;
+  int32_t cg_variant;                  /* gfdtd: CG variant, 0 or 1 as the autotuner
+                                          picked, 2 resident (groups that fit one
+                                          block an SM);
                                           fdtd: E variant + 8 x H variant (0 one
                                           thread per node, 1/2 z-march over 4/16
                                           planes, 3 per-dof coefficient arrays,

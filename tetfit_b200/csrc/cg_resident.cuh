@@ -1,0 +1,155 @@
+// All-to-all sums and on-chip matrix of the resident CG kernels.
+//
+// A system whose rows fit one launch with a few rows a thread is bound by
+// latency: the two inner products of an iteration each end in an exchange of
+// partial sums between every block of the system.  Here a block publishes its
+// partial as one 16-byte record, a double in two 8-byte words of 32 data bits
+// and the 32-bit number of the exchange, so that a record announces itself (an
+// 8-byte word is written at once), and every block polls the records of its
+// system and adds them in a fixed order: one store and one load through L2
+// instead of an atomic counter, a generation word and a read of the partials.
+// Records alternate between two sets: a block overwrites the set of exchange k
+// in exchange k + 2, after it has read every record of k + 1, whose writers had
+// read theirs of k.  Every block of a system is resident (cooperative launch),
+// and a wait is bounded like the grid barrier's (grid_barrier.cuh).
+#pragma once
+#include <cstdint>
+
+#include "grid_barrier.cuh"
+
+namespace tf {
+
+constexpr int kCgVals = 5;     // most values of an exchange
+constexpr int kCgChunks = 10;  // 32-block chunks of a system
+
+struct CgShared {
+  double warp[kCgVals][32];
+  double total[kCgVals * kCgChunks];
+  int dead;
+  alignas(8) uint64_t bar;  // the matrix copy's mbarrier
+};
+
+__device__ __forceinline__ double cg_warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The blocks [first, first + count) of one system.  Every block has a box per
+// value with a record from each block of its system: a record has one reader,
+// which keeps the pollers out of one another's way (148 blocks reading one set
+// of 148 records wait 3 to 5 us for one another in L2, with boxes 2 to 3).
+// box[parity][value][block][producer]
+struct CgExchange {
+  uint4* box;
+  int blocks;       // boxes per value, and records of a box
+  int first, count;
+  int* err;
+  CgShared* sh;
+  uint32_t round;   // number of the next exchange
+
+  // v[] becomes the sums over the system's threads.  With kPublish, global
+  // stores made before the call by any thread of the system are visible to
+  // every thread after it.  False when a wait ran out.
+  template <int NV, bool kPublish>
+  __device__ __forceinline__ bool sum(double (&v)[NV]) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+    const uint32_t k = round++;
+    const int me = blockIdx.x - first, chunks = (count + 31) >> 5;
+#pragma unroll
+    for (int q = 0; q < NV; q++) v[q] = cg_warp_sum(v[q]);
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < NV; q++) sh->warp[q][warp] = v[q];
+    __syncthreads();
+    // a warp adds the block's warps, writes to 32 boxes, then reads 32 records
+    for (int t = warp; t < NV * chunks; t += W) {
+      const int q = t / chunks, i = (t - q * chunks) * 32 + lane;
+      uint4* set = box + ((size_t)(k & 1) * kCgVals + q) * blocks * blocks;
+      double a = __shfl_sync(0xffffffffu, cg_warp_sum(lane < W ? sh->warp[q][lane] : 0.0), 0);
+      if (kPublish) __threadfence();
+      if (i < count) {
+        asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(set + (size_t)(first + i) * blocks +
+                                                                                  me),
+                     "r"((uint32_t)__double2loint(a)), "r"(k), "r"((uint32_t)__double2hiint(a)), "r"(k)
+                     : "memory");
+        const uint4* p = set + (size_t)(first + me) * blocks + i;
+        uint64_t t0 = 0;
+        for (uint32_t n = 0;; n++) {
+          uint32_t x, fx, y, fy;
+          if (kPublish)
+            asm volatile("ld.acquire.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(x), "=r"(fx), "=r"(y), "=r"(fy)
+                         : "l"(p)
+                         : "memory");
+          else
+            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(x), "=r"(fx), "=r"(y), "=r"(fy)
+                         : "l"(p)
+                         : "memory");
+          if (fx == k && fy == k) {
+            a = __hiloint2double((int)y, (int)x);
+            break;
+          }
+          if ((n & 255) == 255) {  // no clock read in a wait that ends at once
+            const uint64_t now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (*(volatile int*)err != 0 || now - t0 > kBarrierLimitNs) {
+              atomicOr(err, kBarrierTimedOut);
+              sh->dead = 1;
+              break;
+            }
+          }
+        }
+      } else {
+        a = 0.0;
+      }
+      a = cg_warp_sum(a);
+      if (lane == 0) sh->total[t] = a;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+      double a = 0.0;
+      for (int c = 0; c < chunks; c++) a += sh->total[q * chunks + c];
+      v[q] = a;
+    }
+    return sh->dead == 0;
+  }
+};
+
+// Bulk copy of global memory into shared memory (sizes and addresses multiples
+// of 16 bytes), one thread; completion is counted on the mbarrier.
+__device__ __forceinline__ uint32_t cg_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cg_bar_init(uint64_t* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cg_smem_u32(bar)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void cg_bar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cg_smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cg_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  constexpr uint32_t kPiece = 32768;
+  for (uint32_t o = 0; o < bytes; o += kPiece) {
+    const uint32_t n = bytes - o < kPiece ? bytes - o : kPiece;
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     cg_smem_u32(dst) + o),
+                 "l"((const char*)src + o), "r"(n), "r"(cg_smem_u32(bar))
+                 : "memory");
+  }
+}
+// bounded wait for the copies of phase 0
+__device__ __forceinline__ bool cg_bar_wait(uint64_t* bar) {
+  for (long it = 0; it < (1L << 22); it++) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(cg_smem_u32(bar))
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+}  // namespace tf

@@ -17,6 +17,7 @@ namespace tf {
 
 namespace {
 
+constexpr int kCgMaxChunksHost = 10;  // kCgMaxChunks of cg_resident.cuh
 constexpr int kTuneSteps = 10;  // 2 warm-up steps, then 4 timed steps per CG variant
 int64_t up32(int64_t n) { return (n + 31) & ~int64_t(31); }
 
@@ -138,6 +139,10 @@ void TetGroup::build(std::vector<TetSim*>& sims, bool release_host) {
     N.col.reserve(room(nn));
     N.val.reserve(room(nn));
   }
+  int sms = 0;
+  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt_.device));
+  int64_t resident_slices = 0;
+  for (TetSim* t : sims) resident_slices += up32((int64_t)t->free_edges_.size()) / 32;
   std::vector<uint16_t> slice_sim, fslice_sim;
   std::vector<double> dt(S), tol(S);
   std::vector<uint8_t> fem(S, 0);
@@ -170,10 +175,14 @@ void TetGroup::build(std::vector<TetSim*>& sims, bool release_host) {
     m.nnz_a = t.A_.val.size();
     // Free rows grouped by stencil: rows whose column offsets (col - row) are
     // the same form a class, classes in order of first appearance, rows of a
-    // class in their own order.  On meshes with repeated local structure the
-    // 32 rows of a slice then gather their j-th entries from consecutive
-    // positions; each class has one row length, so slices carry little
-    // padding.
+    // class in their own order, chunk by chunk of the rows.  On meshes with
+    // repeated local structure the 32 rows of a slice then gather their j-th
+    // entries from consecutive positions; each class has one row length, so
+    // slices carry little padding.  In a group for the resident CG, chunks of
+    // 4096 rows keep what a block gathers close together (40^3 FP32, a solve:
+    // one chunk 316 us, 16384 rows 272, 4096 264, 1024 276); grp_cg ran 1 %
+    // slower with them.
+    const int32_t chunk = resident_slices <= (int64_t)sms * kCgResidentWarps * kCgResidentRows ? 4096 : INT32_MAX;
     std::vector<int32_t> old_of_new(nf), pos(nf), cls(nf);
     auto alen_old = [&](int32_t k) { return t.A_.ptr[k + 1] - t.A_.ptr[k]; };
     {
@@ -187,7 +196,10 @@ void TetGroup::build(std::vector<TetSim*>& sims, bool release_host) {
     }
     std::iota(old_of_new.begin(), old_of_new.end(), 0);
     parallel_stable_sort(old_of_new.begin(), old_of_new.end(), opt_.setup_threads,
-                         [&](int32_t a, int32_t b) { return cls[a] < cls[b]; });
+                         [&](int32_t a, int32_t b) {
+                           const int32_t ca = a / chunk, cb = b / chunk;
+                           return ca != cb ? ca < cb : cls[a] < cls[b];
+                         });
     for (int64_t p = 0; p < nf; p++) pos[old_of_new[p]] = (int32_t)p;
     A.append(
         nfp, nf, [&](int64_t p) { return alen_old(old_of_new[p]); },
@@ -450,8 +462,6 @@ void TetGroup::build(std::vector<TetSim*>& sims, bool release_host) {
     mlp_.loss = fz(1);
     CU(mlp_launch_pack(mlp_.params, mlp_.image, stream_));
     d.mlp_img = mlp_.image;
-    int sms = 0;
-    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt_.device));
     d.guess_blocks = 3 * sms;
     d.tc_blocks = opt_.precision == 1 ? group_guess_tc_blocks<float>(opt_.device)
                                       : group_guess_tc_blocks<double>(opt_.device);
@@ -502,6 +512,10 @@ void TetGroup::build(std::vector<TetSim*>& sims, bool release_host) {
                                    : group_cg_blocks<double>(opt_.device, S, &cg_smem_);
   if (cg_blocks_ < 1) throw CudaError("no co-resident blocks for the cooperative CG kernel");
   partition();
+  if (resident<T>()) {
+    cg_variant_ = kCgResident;
+    tune_pos_ = kTuneSteps;
+  }
   // step_io staging: every member's carrier values of a step in one
   // contiguous H2D buffer, every member's exported sample in one D2H buffer
   std::vector<int> io_src_sim, io_in_off(S + 1, 0);
@@ -652,6 +666,82 @@ void TetGroup::partition() {
   d.err = (int*)dalloc(sizeof(int));
   CU(cudaMemset(d.gbar, 0, 2 * sizeof(unsigned int)));
   CU(cudaMemset(d.err, 0, sizeof(int)));
+}
+
+// The resident CG (grp_cg_resident) when the group's rows fit it: one block an
+// SM, each for one simulation, of about equal work within a simulation, with
+// at most kCgResidentRows rows a thread.  It is faster than grp_cg at every
+// size this takes, to its last (44^3 FP32, 8 rows a thread: 835 us against
+// 955), and gives the same iterates but for the order of the sums.
+template <typename T>
+bool TetGroup::resident() {
+  GroupDev& d = dev_;
+  int sms = 0;
+  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt_.device));
+  sms = std::min(sms, 32 * kCgMaxChunksHost);
+  auto blocks = [&](int64_t per) {
+    int64_t g = 0;
+    for (const Meta& m : meta_) g += (m.nrow_pad / 32 + per - 1) / per;
+    return g;
+  };
+  for (const Meta& m : meta_)
+    if (m.nrow_pad == 0) return false;
+  // rows a thread: as few as keep one block an SM, and then as few warps, but
+  // not fewer than 8: the exchanges of a small system stay between a few blocks
+  int R = 1;
+  while (R <= kCgResidentRows && blocks((int64_t)kCgResidentWarps * R) > sms) R++;
+  if (R > kCgResidentRows) return false;
+  int W = 8;
+  while (W < kCgResidentWarps && blocks((int64_t)W * R) > sms) W++;
+  const int entries = group_resident_entries<T>(opt_.device, R);
+  if (entries == 0) return false;
+  std::vector<int64_t> aptr(d.nrow / 32 + 1);
+  CU(cudaMemcpy(aptr.data(), d.A.ptr, sizeof(int64_t) * aptr.size(), cudaMemcpyDeviceToHost));
+  std::vector<int> sim, first(d.S + 1, 0);
+  std::vector<int64_t> s0;
+  const int64_t per = (int64_t)W * R;
+  for (int s = 0; s < d.S; s++) {
+    // cuts of about equal work (entries, and the row's own passes), with at
+    // most `per` slices a block
+    const int64_t a = meta_[s].roff / 32, n = meta_[s].nrow_pad / 32, g = (n + per - 1) / per;
+    auto work = [&](int64_t sl) { return (double)(aptr[sl] - aptr[a]) / 32 + 4.0 * (double)(sl - a); };
+    first[s] = (int)sim.size();
+    int64_t cut = a;
+    for (int64_t q = 0; q < g; q++) {
+      sim.push_back(s);
+      s0.push_back(cut);
+      int64_t next = cut + 1;
+      while (next < a + n && work(next) < work(a + n) * (double)(q + 1) / (double)g) next++;
+      next = std::min(next, cut + per);
+      // what is left has to fit the blocks left, and each needs a slice
+      next = std::max(next, a + n - (g - 1 - q) * per);
+      cut = std::min(next, a + n - (g - 1 - q));
+    }
+  }
+  first[d.S] = (int)sim.size();
+  s0.push_back(d.nrow / 32);
+  // the copy of A: whole slices from the block's first on, as far as they fit
+  std::vector<int> cached(sim.size(), 0);
+  int most = 0;
+  for (size_t b = 0; b < sim.size(); b++) {
+    for (int64_t sl = s0[b]; sl < s0[b + 1]; sl++)
+      if (aptr[sl + 1] - aptr[s0[b]] <= entries) cached[b] = (int)(aptr[sl + 1] - aptr[s0[b]]);
+    most = std::max(most, cached[b]);
+  }
+  d.res_blocks = (int)sim.size();
+  d.res_warps = W;
+  d.res_rows = R;
+  d.res_entries = most;
+  d.res_cached = (const int*)upload(cached);
+  d.res_sim = (const int*)upload(sim);
+  d.res_s0 = (const int64_t*)upload(s0);
+  d.res_first = (const int*)upload(first);
+  const size_t boxes = (size_t)2 * 5 * sim.size() * sim.size() * 16;
+  d.res_box = (uint4*)dalloc(boxes);
+  CU(cudaMemset(d.res_box, 0, boxes));
+  d.zp = dalloc((size_t)(opt_.warm_start == 3 ? 4 : 2) * (size_t)d.nrow * sizeof(T));
+  cg_blocks_ = d.res_blocks;
+  return true;
 }
 
 // A grid-barrier timeout in the CG kernel leaves the step's results invalid:

@@ -26,6 +26,7 @@
 // Both variants give bitwise identical iterates.
 #include <cuda_runtime.h>
 
+#include "cg_resident.cuh"
 #include "grid_barrier.cuh"
 #include "mlp.cuh"
 #include "mlp_tc.cuh"
@@ -871,6 +872,232 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
     }
 }
 
+// ---------------------------------------------------------------- resident CG
+// grp_cg for groups whose rows fit one block an SM with R rows a thread (see
+// TetGroup::resident).  Every block works for one simulation, keeps its rows'
+// x, r, p and pre in registers and the first entries of its part of A in
+// shared memory (copied once a solve by the bulk copy engine; the rest of A is
+// streamed), and simulations do not wait for one another.  Iteration j:
+//
+//   q = A p_j     a row gathers the pairs (z, p_{j-1}) of its columns, one load
+//                 each, and forms p_j = z + beta p_{j-1} with the rounding
+//                 the column's owner uses
+//   exchange      p.q
+//   x, r, z       in registers; the pair (z, p_j) is stored for the gathers
+//   exchange      r.r, r.z, which also makes the pairs visible
+//
+// Bound by latency.  24^3 FP64 (97 k rows, 146 blocks of 11 warps): an
+// iteration took 20.6 us with grp_cg and takes 11 us, of which the gathers and
+// products 2.3, the exchanges 3.5 and 4.5 us.  9^3 FP64 (5 k rows, 19 blocks):
+// 14.2 -> 6.1 us.  40^3 FP32 (433 k rows, a third of A streamed): 36 -> 22 us.
+// It beat grp_cg at every size it takes (FP64 to 40^3, 952 -> 805 us a solve;
+// FP32 to 44^3, 955 -> 835 us).
+template <typename T>
+struct PairOf;
+template <>
+struct PairOf<float> { typedef float2 type; };
+template <>
+struct PairOf<double> { typedef double2 type; };
+__device__ __forceinline__ float2 make_pair_of(float z, float p) { return make_float2(z, p); }
+__device__ __forceinline__ double2 make_pair_of(double z, double p) { return make_double2(z, p); }
+
+// Sum over a row's entries, in stored order, of val * form(load(col)), CH loads
+// in flight: of the shared copy, whose values are read again behind the
+// loads, or (kShared false) of the matrix itself.
+template <bool kShared, typename T, typename L, typename F>
+__device__ __forceinline__ T resident_dot(const int32_t* col, const T* val, int len, L load, F form) {
+  constexpr int CH = kShared ? 7 : 4;  // 7 and 13 at once measured alike, 8 and 12 slower
+  T s = 0;
+  for (int j0 = 0; j0 < len; j0 += CH) {
+    decltype(load(0)) g[CH];
+    T v[CH];
+    if (kShared) {
+#pragma unroll
+      for (int k = 0; k < CH; k++)
+        if (j0 + k < len) g[k] = load(col[32 * (j0 + k)]);
+    } else {
+      int32_t c[CH];
+#pragma unroll
+      for (int k = 0; k < CH; k++)
+        if (j0 + k < len) {
+          c[k] = ld_stream(col + 32 * (j0 + k));
+          v[k] = ld_stream(val + 32 * (j0 + k));
+        }
+#pragma unroll
+      for (int k = 0; k < CH; k++)
+        if (j0 + k < len) g[k] = load(c[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < CH; k++)
+      if (j0 + k < len) s += (kShared ? val[32 * (j0 + k)] : v[k]) * form(g[k]);
+  }
+  return s;
+}
+
+template <typename T, int R>
+__global__ void __launch_bounds__(32 * kCgResidentWarps, 1) grp_cg_resident(GroupDev d) {
+  typedef typename PairOf<T>::type P;
+  extern __shared__ __align__(128) unsigned char res_raw[];
+  __shared__ CgShared sh;
+  const int s = d.res_sim[blockIdx.x];
+  if (!running(d, s)) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+  const int64_t s0 = d.res_s0[blockIdx.x], s1 = d.res_s0[blockIdx.x + 1];
+  const int64_t e0 = d.A.ptr[s0];
+  const int cached = d.res_cached[blockIdx.x];
+  T* sval = reinterpret_cast<T*>(res_raw);
+  int32_t* scol = reinterpret_cast<int32_t*>(sval + d.res_entries);
+  if (threadIdx.x == 0) {
+    sh.dead = 0;
+    cg_bar_init(&sh.bar);
+    cg_bar_expect(&sh.bar, (uint32_t)cached * (uint32_t)(sizeof(T) + 4));
+    cg_bulk_load(scol, d.A.col + e0, (uint32_t)cached * 4u, &sh.bar);
+    cg_bulk_load(sval, (const T*)d.A.val + e0, (uint32_t)cached * (uint32_t)sizeof(T), &sh.bar);
+  }
+  CgExchange ex{d.res_box, d.res_blocks, d.res_first[s], d.res_first[s + 1] - d.res_first[s], d.err, &sh,
+                (uint32_t)(d.step[s] + 1) * (uint32_t)(2 * d.cg_maxiter + 2)};
+  const T* b = (const T*)d.rhs;
+  T* x = (T*)d.x;
+  const T* pre = (const T*)d.pre;
+  P* zp = (P*)d.zp;
+  const bool dual = d.dual != 0;
+  // this thread's rows: lane of slices s0 + warp, s0 + warp + W, ...
+  int off[R], len[R];
+  T xk[R], rk[R], pk[R], dk[R], qk[R];
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int64_t sl = s0 + warp + (int64_t)k * W;
+    const bool ok = sl < s1;
+    off[k] = ok ? (int)(d.A.ptr[sl] - e0) : 0;
+    len[k] = ok ? (int)((d.A.ptr[sl + 1] - d.A.ptr[sl]) >> 5) : 0;
+    const int64_t i = sl * 32 + lane;
+    xk[k] = ok ? x[i] : (T)0;
+    dk[k] = ok ? pre[i] : (T)0;
+    rk[k] = ok ? b[i] : (T)0;
+    pk[k] = 0;
+    qk[k] = 0;
+  }
+  __syncthreads();  // the mbarrier is initialised
+  bool alive = cg_bar_wait(&sh.bar);
+  if (!alive) atomicOr(d.err, kBarrierTimedOut);
+  auto row_dot = [&](int k, auto load, auto form) -> T {
+    if (off[k] + 32 * len[k] <= cached)
+      return resident_dot<true>(scol + off[k] + lane, sval + off[k] + lane, len[k], load, form);
+    return resident_dot<false>(d.A.col + e0 + off[k] + lane, (const T*)d.A.val + e0 + off[k] + lane, len[k], load, form);
+  };
+  double v5[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  const int64_t i0 = (s0 + warp) * 32 + lane;
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int64_t i = i0 + (int64_t)k * W * 32;
+    if (len[k] == 0) continue;  // a slice of A is never empty (padding rows have their own column)
+    const T bi = rk[k];
+    const T ri = bi - row_dot(k, [&](int32_t c) { return x[c]; }, [](T g) { return g; });
+    const T zi = mulT(dk[k], ri);
+    rk[k] = ri;
+    zp[i] = make_pair_of(zi, (T)0);
+    v5[0] += (double)ri * (double)ri;
+    v5[1] += (double)ri * (double)zi;
+    v5[2] += (double)bi * (double)bi;
+    if (dual) {  // the second start: r_alt = b - A xe was formed by grp_resid_e
+      const T r2 = ((const T*)d.r_alt)[i];
+      const T z2 = mulT(dk[k], r2);
+      zp[d.nrow + i] = make_pair_of(z2, (T)0);
+      v5[3] += (double)r2 * (double)r2;
+      v5[4] += (double)r2 * (double)z2;
+    }
+  }
+  bool sel = false;
+  if (dual) {
+    alive = ex.sum<5, true>(v5) && alive;
+    sel = v5[3] < v5[0];
+  } else {
+    double v3[3] = {v5[0], v5[1], v5[2]};
+    alive = ex.sum<3, true>(v3) && alive;
+    v5[0] = v3[0];
+    v5[1] = v3[1];
+    v5[2] = v3[2];
+  }
+  if (sel) {
+    zp += d.nrow;
+#pragma unroll
+    for (int k = 0; k < R; k++)
+      if (len[k]) {
+        rk[k] = ((const T*)d.r_alt)[i0 + (int64_t)k * W * 32];
+        xk[k] = ((const T*)d.xe)[i0 + (int64_t)k * W * 32];
+      }
+  }
+  const double res0 = sqrt(sel ? v5[3] : v5[0]), bnorm = sqrt(v5[2]), tol = d.tol[s];
+  double res = res0, rz = sel ? v5[4] : v5[1];
+  T beta = 0;
+  int it = 0;
+  auto unmet = [&]() { return d.cg_criterion == 0 ? res / res0 > tol : res > tol * bnorm; };  // NaN (res0 = 0) stops
+  while (alive && it < d.cg_maxiter && unmet()) {
+    const bool first = it == 0;
+    double v1[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      if (len[k] == 0) continue;
+      qk[k] = row_dot(k, [&](int32_t c) { return zp[c]; },
+                      [&](P g) { return p_next<T>(g.x, g.y, beta, first); });
+      pk[k] = p_next<T>(mulT(dk[k], rk[k]), pk[k], beta, first);
+      v1[0] += (double)pk[k] * (double)qk[k];
+    }
+    alive = ex.sum<1, false>(v1);
+    const T alpha = (T)(rz / v1[0]);
+    double v2[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      if (len[k] == 0) continue;
+      xk[k] = fmaT(alpha, pk[k], xk[k]);
+      rk[k] = rk[k] - alpha * qk[k];
+      const T zi = mulT(dk[k], rk[k]);
+      zp[i0 + (int64_t)k * W * 32] = make_pair_of(zi, pk[k]);
+      v2[0] += (double)rk[k] * (double)rk[k];
+      v2[1] += (double)rk[k] * (double)zi;
+    }
+    alive = ex.sum<2, true>(v2) && alive;
+    res = sqrt(v2[0]);
+    beta = (T)(v2[1] / rz);
+    rz = v2[1];
+    it++;
+  }
+  // the solution to x and, scattered, to U (fem groups keep U one step back)
+  T* U = (T*)d.U;
+  T* Uo = (T*)d.Uo;
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    if (len[k] == 0) continue;
+    const int64_t i = i0 + (int64_t)k * W * 32;
+    x[i] = xk[k];
+    const int32_t e = d.free_edge[i];
+    if (e >= 0) {
+      if (Uo) Uo[e] = U[e];
+      U[e] = xk[k];
+    }
+  }
+  if ((int)blockIdx.x == ex.first && threadIdx.x == 0) {
+    const int64_t k = d.stat_off[s] + d.step[s];
+    d.cg_iters[k] = it;
+    d.cg_resid[k] = res / res0;
+    d.cg_limit[k] = unmet() ? 1 : 0;
+    if (d.kept) d.kept[k] = dual && !sel ? 1 : 0;
+  }
+}
+
+// The Dirichlet edges' source values and the step counters (after
+// grp_cg_resident, which scatters the solution itself).
+template <typename T>
+__global__ void __launch_bounds__(kGB) grp_finish(GroupDev d) {
+  const int64_t k = (int64_t)blockIdx.x * kGB + threadIdx.x;
+  if (k < d.ndir) {
+    const int32_t e = d.dir_edge[k];
+    if (d.Uo) ((T*)d.Uo)[e] = ((const T*)d.U)[e];
+    ((T*)d.U)[e] = ((const T*)d.src)[e];
+  }
+  if (k < d.S && d.step[k] < d.nsteps[k]) d.step[k] += 1;
+}
+
 // Leapfrog energy of member s in the state after a step, (U^n, B^{n-1/2}):
 // W^n = 0.5 U^n.E.U^n + 0.5 B^{n-1/2}.N.B^{n+1/2}, with B^{n+1/2} =
 // B^{n-1/2} - dt C U^n recomputed per gathered face (what the next step's
@@ -1003,6 +1230,41 @@ int group_cg_blocks(int device, int S, size_t* smem) {
   return (a < b ? a : b) * sms;
 }
 
+template <typename T>
+static void (*resident_kernel(int rows))(GroupDev) {
+  switch (rows) {
+    case 1: return grp_cg_resident<T, 1>;
+    case 2: return grp_cg_resident<T, 2>;
+    case 3: return grp_cg_resident<T, 3>;
+    case 4: return grp_cg_resident<T, 4>;
+    case 5: case 6: return grp_cg_resident<T, 6>;
+    default: return grp_cg_resident<T, 8>;
+  }
+}
+
+// Matrix entries a resident CG block's shared memory holds (a multiple of
+// 32), 0 when the kernel cannot be launched with that much.
+template <typename T>
+int group_resident_entries(int device, int rows) {
+  int most = 0, per_sm = 0;
+  cudaFuncAttributes fa{};
+  auto k = resident_kernel<T>(rows);
+  if (cudaFuncGetAttributes(&fa, k) != cudaSuccess ||
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+    return 0;
+  const int n = (most - (int)fa.sharedSizeBytes) / (int)((sizeof(T) + 4) * 32) * 32;
+  const int bytes = n * (int)(sizeof(T) + 4);
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kCgResidentWarps, bytes) != cudaSuccess ||
+      per_sm < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+template int group_resident_entries<float>(int, int);
+template int group_resident_entries<double>(int, int);
+
 // Resident CTAs of the tensor-core guess kernel over the whole GPU, from its
 // registers and shared memory against the SM's limits, capped at the 8 CTAs
 // whose 64 TMEM columns each fill the SM's 512 (the runtime's occupancy
@@ -1067,19 +1329,27 @@ cudaError_t group_launch_step(const GroupDev& d, int cg_blocks, int cg_variant, 
   }
   if (ev) cudaEventRecord(ev[2], st);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cg_blocks);
-  cfg.blockDim = dim3(cg_threads<T>());
-  cfg.dynamicSmemBytes = smem;
+  const bool resident = cg_variant == kCgResident;
+  cfg.gridDim = dim3(resident ? d.res_blocks : cg_blocks);
+  cfg.blockDim = dim3(resident ? 32 * d.res_warps : cg_threads<T>());
+  cfg.dynamicSmemBytes = resident ? (sizeof(T) + 4) * (size_t)d.res_entries : smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t err = cg_variant == 0 ? cudaLaunchKernelEx(&cfg, grp_cg<T, true>, d)
-                                    : cudaLaunchKernelEx(&cfg, grp_cg<T, false>, d);
+  cudaError_t err = resident ? cudaLaunchKernelEx(&cfg, resident_kernel<T>(d.res_rows), d)
+                    : cg_variant == 0 ? cudaLaunchKernelEx(&cfg, grp_cg<T, true>, d)
+                                      : cudaLaunchKernelEx(&cfg, grp_cg<T, false>, d);
   if (err != cudaSuccess) return err;
   if (ev) cudaEventRecord(ev[3], st);
+  if (resident) {
+    grp_finish<T><<<gblk(d.ndir > d.S ? d.ndir : d.S), kGB, 0, st>>>(d);
+    if (ev) cudaEventRecord(ev[4], st);
+    if (ev) cudaEventRecord(ev[5], st);
+    return cudaGetLastError();
+  }
   grp_scatter<T><<<gblk(d.nrow > d.ndir ? d.nrow : d.ndir), kGB, 0, st>>>(d);
   if (ev) cudaEventRecord(ev[4], st);
   grp_bump<<<(d.S + 127) / 128, 128, 0, st>>>(d);

@@ -23,6 +23,8 @@
 // segments, and every inner product is summed per segment, then per
 // simulation in segment order, so results do not depend on timing.
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace tf {
@@ -113,6 +115,16 @@ struct GroupDev {
   double* part = nullptr;        // [nseg][kCgPart]
   unsigned int* gbar = nullptr;  // grid barrier: arrivals, generation
   int* err = nullptr;            // set when a grid barrier wait ran out of time
+  // resident CG (grp_cg_resident): block b works for simulation res_sim[b] on
+  // the slices [res_s0[b], res_s0[b + 1]); simulation s has the blocks
+  // [res_first[s], res_first[s + 1])
+  int res_blocks = 0, res_warps = 0, res_rows = 0, res_entries = 0;  // rows a thread, most copied entries of a block
+  const int* res_sim = nullptr;
+  const int64_t* res_s0 = nullptr;
+  const int* res_first = nullptr;
+  const int* res_cached = nullptr;  // entries of A a block copies (whole slices)
+  uint4* res_box = nullptr;      // exchange boxes (cg_resident.cuh)
+  void* zp = nullptr;            // pairs (z, p) of the rows, once more for the second start of warm_start 3
   int cg_maxiter = 100, cg_criterion = 0, warm_start = 0;
   // learned warm start (warm_start 3): the network's guess goes to x, the
   // quadratic extrapolation to xe; with dual set, the CG starts from the one
@@ -163,6 +175,11 @@ cudaError_t group_launch_step(const GroupDev& d, int cg_blocks, int cg_variant, 
                               cudaEvent_t* ev);
 template <typename T>
 int group_cg_blocks(int device, int S, size_t* smem);
+constexpr int kCgResident = 2;      // CG variant: 0 fused, 1 three barriers, 2 resident
+constexpr int kCgResidentWarps = 16;  // most warps of a block: 128 registers a thread hold up to 8 rows
+constexpr int kCgResidentRows = 8;    // most rows of a thread
+template <typename T>
+int group_resident_entries(int device, int rows);
 // step_io: this step's carrier values (staging, contiguous) into each
 // running member's carrier row
 cudaError_t group_launch_io_carriers(const GroupDev& d, const double* in, cudaStream_t st);
