@@ -32,6 +32,8 @@ namespace tf {
 template <typename T>
 cudaError_t tet_launch_step(const DevPtrs& d, cudaStream_t st, cudaEvent_t* ev);
 template <typename T>
+cudaError_t tet_launch_export(const void* v, const int32_t* where, double* out, int n, cudaStream_t st);
+template <typename T>
 void tet_launch_initial_probes(const DevPtrs& d, cudaStream_t st);
 template <typename T>
 cudaError_t tet_launch_energy(const DevPtrs& d, DevPtrs d_cg, int cg_blocks, const int32_t* ie, int ni,
@@ -363,8 +365,7 @@ uint64_t TetSim::device_bytes() const { return group_ ? group_->device_bytes() :
 double TetSim::last_step_ms() const { return group_ ? group_->last_step_ms() : last_ms_; }
 int TetSim::kernels_per_step() const {
   if (group_) return group_->kernels_per_step();
-  const int np = probe_tet_.empty() ? 0 : 1;
-  return 6 + np + (src_edge_.empty() ? 0 : 1) + (dp_.nq > 0 ? 1 : 0) + (dp_.nfe > 0 ? 1 : 0);
+  return 4 + (dp_.nq > 0 ? 1 : 0) + (dp_.nfe > 0 ? 1 : 0);
 }
 
 void TetSim::release_host() {
@@ -382,6 +383,7 @@ void TetSim::release_host() {
 
 TetSim::~TetSim() {
   group_.reset();
+  if (graph_) cudaGraphExecDestroy(graph_);
   if (pinned_) cudaFreeHost(pinned_);
   for (void* p : allocs_) cudaFree(p);
   if (ev0_) cudaEventDestroy(ev0_);
@@ -1761,6 +1763,34 @@ void TetSim::build_sources() {
   }
 }
 
+// Rows of a matrix in chunks of 4096, rows whose column offsets (col - row)
+// are the same side by side within a chunk, each form in its own order.  The
+// forms are told apart by a hash of the offsets; equal hashes of different
+// forms would only mix them.
+static std::vector<int32_t> stencil_order(const HostCsr& m, int threads) {
+  const int64_t n = (int64_t)m.ptr.size() - 1;
+  std::vector<uint64_t> form(n);
+  parallel_for(n, threads, [&](int64_t a, int64_t b) {
+    for (int64_t i = a; i < b; i++) {
+      uint64_t h = 0xcbf29ce484222325ull;
+      for (int64_t k = m.ptr[i]; k < m.ptr[i + 1]; k++) {
+        h = (h ^ (uint32_t)(m.col[k] - (int32_t)i)) * 0x100000001b3ull;
+        h ^= h >> 29;
+      }
+      form[i] = h;
+    }
+  });
+  std::vector<int32_t> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  constexpr int64_t kChunk = 4096;
+  parallel_for((n + kChunk - 1) / kChunk, threads, [&](int64_t a, int64_t b) {
+    for (int64_t c = a; c < b; c++)
+      std::stable_sort(order.begin() + c * kChunk, order.begin() + std::min(n, (c + 1) * kChunk),
+                       [&](int32_t x, int32_t y) { return form[x] < form[y]; });
+  }, 1);
+  return order;
+}
+
 void TetSim::alloc_and_upload() {
   CU(cudaSetDevice(opt_.device));
   int major = 0;
@@ -1797,38 +1827,127 @@ void TetSim::alloc_and_upload() {
   };
   DevPtrs& d = dp_;
   const size_t NE = edges_.size(), NF = faces_.size();
+  const int nth = opt_.setup_threads;
   d.nE = (int)NE;
   d.nF = (int)NF;
   d.dt = dt_;
   d.U = zeros(NE); d.F = zeros(NF); d.B = zeros(NF); d.cu = zeros(NF); d.cf = zeros(NE);
   d.I = zeros(NE); d.cb = zeros(NE);
-  d.fte = (const int32_t*)up(fte_.data(), NF * 3 * 4);
+  // device numbering: chunks of 4096 rows, rows of one form (the same column
+  // offsets) side by side within them, as in the group engine's layout
+  const std::vector<int32_t> e_old = stencil_order(H_, nth), f_old = stencil_order(N_, nth);
+  edge_new_.resize(NE);
+  face_new_.resize(NF);
+  parallel_for((int64_t)NE, nth, [&](int64_t a, int64_t b) {
+    for (int64_t i = a; i < b; i++) edge_new_[e_old[i]] = (int32_t)i;
+  });
+  parallel_for((int64_t)NF, nth, [&](int64_t a, int64_t b) {
+    for (int64_t i = a; i < b; i++) face_new_[f_old[i]] = (int32_t)i;
+  });
+  dedge_new_ = (const int32_t*)up(edge_new_.data(), NE * 4);
+  dface_new_ = (const int32_t*)up(face_new_.data(), NF * 4);
+  dexport_ = (double*)dalloc(std::max(NE, NF) * 8);
   {
-    std::vector<int32_t> cc(Ct_.col.size());
-    for (size_t k = 0; k < cc.size(); k++) cc[k] = Ct_.val[k] < 0 ? (int32_t)((uint32_t)Ct_.col[k] | 0x80000000u) : Ct_.col[k];
-    d.ct_ptr = (const int64_t*)up(Ct_.ptr.data(), Ct_.ptr.size() * 8);
-    d.ct_col = (const int32_t*)up(cc.data(), cc.size() * 4);
+    std::vector<int32_t, default_init_allocator<int32_t>> fte(3 * NF);
+    parallel_for((int64_t)NF, nth, [&](int64_t a, int64_t b) {
+      for (int64_t i = a; i < b; i++)
+        for (int k = 0; k < 3; k++) fte[k * NF + i] = edge_new_[fte_[f_old[i]][k]];
+    });
+    d.fte = (const int32_t*)up(fte.data(), fte.size() * 4);
+    std::vector<uint8_t> upd(NE);
+    for (size_t i = 0; i < NE; i++) upd[i] = H_.ptr[e_old[i] + 1] > H_.ptr[e_old[i]];
+    d.edge_upd = (const uint8_t*)up(upd.data(), NE);
+    CU(cudaStreamSynchronize(stream_));
   }
-  auto upcsr = [&](const HostCsr& m, const int64_t*& ptr, const int32_t*& col, const void*& val) {
-    ptr = (const int64_t*)up(m.ptr.data(), m.ptr.size() * 8);
-    col = (const int32_t*)up(m.col.data(), m.col.size() * 4);
-    val = upT(m.val);
+  // 32-row slices of a matrix's rows in the device numbering
+  auto sell = [&](const HostCsr& m, const std::vector<int32_t>& row_old, const std::vector<int32_t>& col_new,
+                  bool values) {
+    const int64_t n = (int64_t)row_old.size(), ns = (n + 31) / 32;
+    std::vector<int64_t> ptr(ns + 1, 0);
+    auto len = [&](int64_t i) { return m.ptr[row_old[i] + 1] - m.ptr[row_old[i]]; };
+    parallel_for(ns, nth, [&](int64_t s0, int64_t s1) {
+      for (int64_t s = s0; s < s1; s++)
+        for (int64_t i = 32 * s; i < std::min(n, 32 * s + 32); i++) ptr[s + 1] = std::max<int64_t>(ptr[s + 1], 32 * len(i));
+    }, 64);
+    for (int64_t s = 0; s < ns; s++) ptr[s + 1] += ptr[s];
+    std::vector<int32_t, default_init_allocator<int32_t>> col(ptr[ns]);
+    std::vector<float, default_init_allocator<float>> vf(values && f32 ? ptr[ns] : 0);
+    std::vector<double, default_init_allocator<double>> vd(values && !f32 ? ptr[ns] : 0);
+    parallel_for(ns, nth, [&](int64_t s0, int64_t s1) {
+      for (int64_t s = s0; s < s1; s++) {
+        int64_t k0[32], nr[32];
+        for (int l = 0; l < 32; l++) {
+          const int64_t i = 32 * s + l;
+          k0[l] = i < n ? m.ptr[row_old[i]] : 0;
+          nr[l] = i < n ? len(i) : 0;
+        }
+        const int64_t w = (ptr[s + 1] - ptr[s]) / 32;
+        for (int64_t j = 0; j < w; j++)
+          for (int l = 0; l < 32; l++) {
+            const int64_t q = ptr[s] + 32 * j + l;
+            const bool real = j < nr[l];
+            const int32_t c = real || nr[l] ? col_new[m.col[k0[l] + (real ? j : 0)]] : 0;
+            const double v = real ? m.val[k0[l] + j] : 0.0;
+            if (values) {
+              col[q] = c;
+              if (f32) vf[q] = (float)v;
+              else vd[q] = v;
+            } else {
+              col[q] = !real ? kNoFace : v < 0 ? (int32_t)((uint32_t)c | 0x80000000u) : c;
+            }
+          }
+      }
+    }, 64);
+    TetSell o;
+    o.ptr = (const int64_t*)up(ptr.data(), ptr.size() * 8);
+    o.col = (const int32_t*)up(col.data(), col.size() * 4);
+    if (values) o.val = f32 ? up(vf.data(), vf.size() * 4) : up(vd.data(), vd.size() * 8);
+    CU(cudaStreamSynchronize(stream_));
+    return o;
   };
-  upcsr(N_, d.n_ptr, d.n_col, d.n_val);
-  upcsr(H_, d.h_ptr, d.h_col, d.h_val);
-  if (!nr_.empty()) d.n_r = upT(nr_);
+  d.Ct = sell(Ct_, e_old, face_new_, false);
+  d.N = sell(N_, f_old, face_new_, true);
+  d.H = sell(H_, e_old, edge_new_, true);
+  auto upcsr = [&](const HostCsr& m, const std::vector<int32_t>* col_new, const int64_t*& ptr, const int32_t*& col,
+                   const void*& val) {
+    std::vector<int32_t> c(m.col.begin(), m.col.end());
+    if (col_new)
+      for (int32_t& q : c) q = (*col_new)[q];
+    ptr = (const int64_t*)up(m.ptr.data(), m.ptr.size() * 8);
+    col = (const int32_t*)up(c.data(), c.size() * 4);
+    val = upT(m.val);
+    CU(cudaStreamSynchronize(stream_));
+  };
+  auto reordered = [&](const std::vector<double>& v, const std::vector<int32_t>& old) {
+    std::vector<double> o(v.size());
+    for (size_t i = 0; i < o.size(); i++) o[i] = v[old[i]];
+    return o;
+  };
+  auto renumbered = [&](std::vector<int32_t> v, const std::vector<int32_t>& to) {
+    for (int32_t& q : v) q = to[q];
+    return v;
+  };
+  if (!nr_.empty()) {
+    const auto r = reordered(nr_, f_old);
+    d.n_r = upT(r);
+    CU(cudaStreamSynchronize(stream_));
+  }
   if (dga_frac_) {
-    d.h_p = upT(hp_);
+    const auto hp = reordered(hp_, e_old);
+    d.h_p = upT(hp);
+    CU(cudaStreamSynchronize(stream_));
     d.nq = (int)q_size_;
     d.nfe = (int)fe_edge_.size();
     if (d.nq > 0) {
-      upcsr(Q_, d.q_ptr, d.q_col, d.q_val);
-      upcsr(Mq_, d.mq_ptr, d.mq_col, d.mq_val);
+      upcsr(Q_, nullptr, d.q_ptr, d.q_col, d.q_val);
+      upcsr(Mq_, &edge_new_, d.mq_ptr, d.mq_col, d.mq_val);
       d.Uc = zeros(q_size_);
       d.Uc_old = zeros(q_size_);
     }
     if (d.nfe > 0) {
-      d.fe_edge = (const int32_t*)up(fe_edge_.data(), fe_edge_.size() * 4);
+      const auto fe = renumbered(fe_edge_, edge_new_);
+      d.fe_edge = (const int32_t*)up(fe.data(), fe.size() * 4);
+      CU(cudaStreamSynchronize(stream_));
       d.fe_a = (const int32_t*)up(fe_a_.data(), fe_a_.size() * 4);
       d.fe_b = (const int32_t*)up(fe_b_.data(), fe_b_.size() * 4);
     }
@@ -1836,7 +1955,9 @@ void TetSim::alloc_and_upload() {
   const size_t nsrc = src_labels_.size();
   d.nse = (int)src_edge_.size();
   d.nsrc = (int)nsrc;
-  d.se_edge = (const int32_t*)up(src_edge_.data(), src_edge_.size() * 4);
+  std::vector<int32_t> edge_src(NE, -1);
+  for (size_t k = 0; k < src_edge_.size(); k++) edge_src[edge_new_[src_edge_[k]]] = (int32_t)k;
+  d.edge_src = (const int32_t*)up(edge_src.data(), NE * 4);
   d.se_kind = (const int8_t*)up(src_kind_e_.data(), src_kind_e_.size());
   d.se_begin = (const int*)up(src_begin_.data(), src_begin_.size() * 4);
   d.pair_src = (const int*)up(pair_src_.data(), pair_src_.size() * 4);
@@ -1859,8 +1980,8 @@ void TetSim::alloc_and_upload() {
   std::vector<int32_t> pe(6 * np), pf(4 * np);
   for (size_t p = 0; p < np; p++) {
     auto el = vol_edges(probe_tet_[p]);
-    for (int q = 0; q < 6; q++) pe[6 * p + q] = el[q];
-    for (int q = 0; q < 4; q++) pf[4 * p + q] = vtf_[probe_tet_[p]][q];
+    for (int q = 0; q < 6; q++) pe[6 * p + q] = edge_new_[el[q]];
+    for (int q = 0; q < 4; q++) pf[4 * p + q] = face_new_[vtf_[probe_tet_[p]][q]];
   }
   d.np = (int)np;
   d.p_edges = (const int32_t*)up(pe.data(), pe.size() * 4);
@@ -1869,8 +1990,8 @@ void TetSim::alloc_and_upload() {
   d.p_hf = (const double*)up(probe_hf_.data(), probe_hf_.size() * 8);
   d.samples = (double*)dalloc((size_t)nslots_ * np * 6 * 8);
   d.slot_of_step = (const int*)up(slot_of_step_.data(), slot_of_step_.size() * 4);
-  d.step = (int*)dalloc(sizeof(int));
-  CU(cudaMemsetAsync(d.step, 0, sizeof(int), stream_));
+  d.step = (int*)dalloc(2 * sizeof(int));
+  CU(cudaMemsetAsync(d.step, 0, 2 * sizeof(int), stream_));
   CU(cudaHostAlloc((void**)&pinned_, (nsrc + 6 * np + 1) * sizeof(double), cudaHostAllocDefault));
   // initial state (t = 0 sources, Discretization.hpp:671-791)
   auto put_state = [&](void* dst, const std::vector<double>& v) {
@@ -1881,8 +2002,9 @@ void TetSim::alloc_and_upload() {
       CU(cudaStreamSynchronize(stream_));
     }
   };
-  put_state(d.U, init_U_);
-  put_state(d.I, init_I_);
+  const auto u0 = reordered(init_U_, e_old), i0 = reordered(init_I_, e_old);
+  put_state(d.U, u0);
+  put_state(d.I, i0);
   if (f32) tet_launch_initial_probes<float>(d, stream_);
   else tet_launch_initial_probes<double>(d, stream_);
   CU(cudaGetLastError());
@@ -1905,8 +2027,21 @@ uint64_t TetSim::step(uint64_t n) {
   }
   if (step_ + n > nsteps_) n = nsteps_ - step_;
   if (n == 0) { last_ms_ = 0; return 0; }
+  // every step launches the same kernels with the same arguments: runs of glen
+  // steps replay one captured graph, captured before the timed region opens
+  const int glen = opt_.graph_steps > 0 ? opt_.graph_steps : 16;
+  if (glen > 1 && n >= (uint64_t)glen && !graph_) {
+    cudaGraph_t g;
+    CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+    launch_steps(glen, nullptr);
+    CU(cudaStreamEndCapture(stream_, &g));
+    CU(cudaGraphInstantiate(&graph_, g, 0));
+    CU(cudaGraphDestroy(g));
+  }
   CU(cudaEventRecord(ev0_, stream_));
-  launch_steps((int)n, nullptr);
+  uint64_t left = n;
+  for (; graph_ && left >= (uint64_t)glen; left -= glen) CU(cudaGraphLaunch(graph_, stream_));
+  launch_steps((int)left, nullptr);
   CU(cudaEventRecord(ev1_, stream_));
   CU(cudaEventSynchronize(ev1_));
   float ms = 0;
@@ -1991,24 +2126,19 @@ void TetSim::probe_points(double* xyz, uint64_t* cells, size_t cap) const {
   }
 }
 
-static void fetch(const void* d, size_t n, bool f32, double* out) {
-  if (!out) return;
-  if (!f32) {
-    CU(cudaMemcpy(out, d, n * 8, cudaMemcpyDeviceToHost));
-    return;
-  }
-  std::vector<float> tmp(n);
-  CU(cudaMemcpy(tmp.data(), d, n * 4, cudaMemcpyDeviceToHost));
-  for (size_t i = 0; i < n; i++) out[i] = tmp[i];
-}
-
 void TetSim::get_state(double* U, double* B, double* F) {
   if (group_) return group_->get_state(0, U, B, F);
-  const bool f32 = opt_.precision == 1;
-  CU(cudaStreamSynchronize(stream_));
-  fetch(dp_.U, edges_.size(), f32, U);
-  fetch(dp_.B, faces_.size(), f32, B);
-  fetch(dp_.F, faces_.size(), f32, F);
+  // dga: renumbered and widened on the GPU, one field at a time
+  auto get = [&](const void* v, const int32_t* where, size_t n, double* out) {
+    if (!out || !n) return;
+    CU(opt_.precision == 1 ? tet_launch_export<float>(v, where, dexport_, (int)n, stream_)
+                           : tet_launch_export<double>(v, where, dexport_, (int)n, stream_));
+    CU(cudaMemcpyAsync(out, dexport_, n * 8, cudaMemcpyDeviceToHost, stream_));
+    CU(cudaStreamSynchronize(stream_));
+  };
+  get(dp_.U, dedge_new_, edges_.size(), U);
+  get(dp_.B, dface_new_, faces_.size(), B);
+  get(dp_.F, dface_new_, faces_.size(), F);
 }
 
 void TetSim::set_state(const double* U, const double* F) {
@@ -2016,16 +2146,18 @@ void TetSim::set_state(const double* U, const double* F) {
   if (U && q_size_ > 0)
     throw UnsupportedError("tf_set_state: a dga run with fractured edges keeps node-star fractions that U does not fix");
   const bool f32 = opt_.precision == 1;
-  auto put = [&](void* dst, const double* src, size_t n) {
+  auto put = [&](void* dst, const double* src, const std::vector<int32_t>& where) {
     if (!src) return;
-    if (!f32) CU(cudaMemcpy(dst, src, n * 8, cudaMemcpyHostToDevice));
-    else {
-      std::vector<float> t(src, src + n);
-      CU(cudaMemcpy(dst, t.data(), n * 4, cudaMemcpyHostToDevice));
-    }
+    const size_t n = where.size();
+    auto set = [&](auto tmp) {
+      for (size_t i = 0; i < n; i++) tmp[where[i]] = src[i];
+      CU(cudaMemcpy(dst, tmp.data(), n * sizeof(tmp[0]), cudaMemcpyHostToDevice));
+    };
+    if (f32) set(std::vector<float>(n));
+    else set(std::vector<double>(n));
   };
-  put(dp_.U, U, edges_.size());
-  put(dp_.F, F, faces_.size());
+  put(dp_.U, U, edge_new_);
+  put(dp_.F, F, face_new_);
 }
 
 void TetSim::get_flux(double* flux, size_t cap, size_t* n) const {
@@ -2134,6 +2266,7 @@ double TetSim::dga_energy() {
     c.cg_maxiter = 5000;
     c.cg_criterion = 1;
     en_n_ = ni;
+    for (int32_t& e : ie) e = edge_new_[e];  // the matrix above is by rank, the fields are in the device numbering
     en_edges_ = (int32_t*)up(ie.data(), ie.size() * 4);
     const size_t nparts = 2 * (((size_t)ni + 255) / 256 + 1) + ((faces_.size() + 255) / 256 + 1);
     en_part_ = (double*)dalloc(nparts * 8);

@@ -177,6 +177,10 @@ class TetSim : public Sim {
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   std::vector<void*> allocs_;
   DevPtrs dp_{};
+  std::vector<int32_t> edge_new_, face_new_;       // dga: device number of an edge and a face
+  const int32_t *dedge_new_ = nullptr, *dface_new_ = nullptr;
+  double* dexport_ = nullptr;                      // a field on its way to the host
+  cudaGraphExec_t graph_ = nullptr;
   double* pinned_ = nullptr;
   // gfdtd runs on the group engine (a group of one simulation)
   std::unique_ptr<TetGroup> group_;

@@ -2,19 +2,19 @@
 // standalone CG solve of the C ABI.  (gfdtd simulations run on the group
 // engine, tet_group_kernels.cu, also when a simulation is alone.)
 //
-//   tet_curl_u        cu = C U (3 signed edges per face), B -= dt cu
-//                     (Discretization.hpp:902-916)
-//   tet_nmul          F = R F - dt N cu (:917-918; R = 1 without magnetic
-//                     losses)
-//   tet_curl_f        cf = C^T F + Ctb Fb - I (:878-879)
+//   tet_curl_f        cf = C^T F + Ctb Fb - I, with the step's source values:
+//                     E values to U, boundary dual-edge H sources, currents
+//                     (:821-868, :878-879)
 //   tet_h_update      U = P U + dt H cf on interior edges (P = 1 when
-//                     lossless), boundary flux (:887-894)
+//                     lossless), boundary flux partials (:887-894)
 //   tet_frac_update   U_c = Q U_c_old + dt Mq cf: node-star fractions of the
 //                     fractured edges (:891)
 //   tet_frac_gather   U = sum of a fractured edge's two fractions (:892), flux
-//   tet_sources       source edges from the carrier table: E values, boundary
-//                     dual-edge H sources, currents (:821-868)
-//   tet_probes        Whitney E and face-flux H at probe points (:3768-3897)
+//   tet_curl_u        cu = C U (3 signed edges per face), B -= dt cu
+//                     (:902-916); flux sum
+//   tet_nmul          F = R F - dt N cu (:917-918; R = 1 without magnetic
+//                     losses); Whitney E and face-flux H at the probe points
+//                     (:3768-3897); step counter
 //   tet_cg            persistent cooperative Jacobi-PCG on a CSR system
 //                     (ConjugateGradientSolver.hpp:52-103): SpMV, dots and
 //                     axpys fused, FP64 reductions in a fixed order, a hard
@@ -51,58 +51,136 @@ __device__ double block_sum(double v, double* sh) {
   return sh[32];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kBlock) tet_curl_u(DevPtrs d) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= d.nF) return;
-  const T* U = (const T*)d.U;
-  const int32_t* e = d.fte + 3 * (int64_t)f;
-  T c = U[e[0]] - U[e[1]] + U[e[2]];
-  ((T*)d.cu)[f] = c;
-  T* B = (T*)d.B;
-  B[f] = B[f] - (T)d.dt * c;
+// A step is four launches (six with fractured edges), each waiting for the one
+// before it (programmatic dependent launch) with its matrix row's first loads
+// already made.  The matrices are SELL-32 in the device numbering: edges and
+// faces ordered by the column offsets of their H and N rows, so that a warp
+// reads one entry slot with one 128- or 256-byte load and gathers from
+// neighbouring places.  Bound by launch latency up to some 10^5 edges, then by
+// the matrices' bytes.  24^3 FP64 (102 k edges): 49 us a step with eight
+// launches, one thread walking one CSR row each, 14.4 us now; 36^3 FP32 (0.12 GB a
+// step, half of it H) 83 us, 30 us now.
+__device__ __forceinline__ int32_t ld_index(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_value(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_value(const double* p) {
+  double v;
+  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
 }
 
-// F -= dt N cu
-template <typename T>
-__global__ void __launch_bounds__(kBlock) tet_nmul(DevPtrs d) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= d.nF) return;
-  const T* x = (const T*)d.cu;
+// Sum over row i's entries in stored order of val * x[col]; ready() runs
+// between the first entries' loads and their gathers.
+template <typename T, int CH, typename W>
+__device__ __forceinline__ T tet_row(const TetSell& m, int i, const T* x, W ready) {
+  const int64_t b = m.ptr[i >> 5];
+  const int len = (int)((m.ptr[(i >> 5) + 1] - b) >> 5);
+  const int32_t* col = m.col + b + (i & 31);
+  const T* val = (const T*)m.val + b + (i & 31);
   T s = 0;
-  for (int64_t k = d.n_ptr[f]; k < d.n_ptr[f + 1]; k++) s += ld<T>(d.n_val, k) * x[d.n_col[k]];
-  T* F = (T*)d.F;
-  F[f] = d.n_r ? ((const T*)d.n_r)[f] * F[f] - (T)d.dt * s : F[f] - (T)d.dt * s;
-}
-
-template <typename T>
-__device__ __forceinline__ T ctf(const DevPtrs& d, int e) {
-  const T* F = (const T*)d.F;
-  T s = 0;
-  for (int64_t k = d.ct_ptr[e]; k < d.ct_ptr[e + 1]; k++) {
-    const int32_t c = d.ct_col[k];
-    const T v = F[c & 0x7fffffff];
-    s = c < 0 ? s - v : s + v;
+  for (int j0 = 0; j0 < len || j0 == 0; j0 += CH) {
+    int32_t c[CH];
+    T v[CH];
+#pragma unroll
+    for (int k = 0; k < CH; k++)
+      if (j0 + k < len) {
+        c[k] = ld_index(col + 32 * (j0 + k));
+        v[k] = ld_value(val + 32 * (j0 + k));
+      }
+    if (j0 == 0) ready();
+#pragma unroll
+    for (int k = 0; k < CH; k++)
+      if (j0 + k < len) s += v[k] * x[c[k]];
   }
   return s;
 }
 
-template <typename T>
+__device__ __forceinline__ double source_value(const DevPtrs& d, int s, int row) {
+  double v[3] = {0.0, 0.0, 0.0};
+  for (int p = d.se_begin[s]; p < d.se_begin[s + 1]; p++) {
+    const int si = d.pair_src[p];
+    double ret = d.src_amp[si] * d.carrier[(int64_t)row * d.nsrc + si];
+    ret *= d.pair_fac[4 * p + 0];
+    ret *= d.pair_fac[4 * p + 1];
+    ret *= d.pair_fac[4 * p + 2];
+    ret *= d.pair_fac[4 * p + 3];
+    const int a = d.pair_dir[p];
+    if (a == 0) v[0] += ret;
+    else if (a == 1) v[1] += ret;
+    else v[2] += ret;
+  }
+  const double* w = d.se_vec + 3 * (int64_t)s;
+  return d.se_post[s] * ((v[0] * w[0] + v[1] * w[1]) + v[2] * w[2]);
+}
+
+// kStep: the step's source values first (an H-source edge's cb and a current
+// edge's I are rewritten every step; every other edge's stay zero)
+template <typename T, bool kStep>
 __global__ void __launch_bounds__(kBlock) tet_curl_f(DevPtrs d) {
+  constexpr int CH = 6;
+  if (kStep) cudaTriggerProgrammaticLaunchCompletion();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= d.nE) return;
-  ((T*)d.cf)[e] = ctf<T>(d, e) + ((const T*)d.cb)[e] - ((const T*)d.I)[e];
+  const T* F = (const T*)d.F;
+  const bool ok = e < d.nE;
+  int64_t b = 0;
+  int len = 0, src = -1;
+  int32_t c[CH];
+  if (ok) {
+    b = d.Ct.ptr[e >> 5];
+    len = (int)((d.Ct.ptr[(e >> 5) + 1] - b) >> 5);
+    b += e & 31;
+    src = d.edge_src[e];
+#pragma unroll
+    for (int k = 0; k < CH; k++) c[k] = k < len ? ld_index(d.Ct.col + b + 32 * k) : kNoFace;
+  }
+  if (kStep) cudaGridDependencySynchronize();
+  if (!ok) return;
+  T s = 0;
+  for (int j0 = 0;;) {
+    T f[CH];
+#pragma unroll
+    for (int k = 0; k < CH; k++) f[k] = c[k] != kNoFace ? F[c[k] & 0x7fffffff] : (T)0;
+#pragma unroll
+    for (int k = 0; k < CH; k++)
+      if (c[k] != kNoFace) s = c[k] < 0 ? s - f[k] : s + f[k];
+    j0 += CH;
+    if (j0 >= len) break;
+#pragma unroll
+    for (int k = 0; k < CH; k++) c[k] = j0 + k < len ? ld_index(d.Ct.col + b + 32 * (j0 + k)) : kNoFace;
+  }
+  T cb = ((const T*)d.cb)[e], cur = ((const T*)d.I)[e];
+  if (kStep && src >= 0) {
+    const T v = (T)source_value(d, src, d.step[0]);
+    const int kind = d.se_kind[src];
+    if (kind == 1) {
+      ((T*)d.U)[e] = v;
+    } else if (kind == 2) {
+      ((T*)d.cb)[e] = cb = v;
+    } else if (kind == 3) {
+      ((T*)d.I)[e] = cur = v;
+    }
+  }
+  ((T*)d.cf)[e] = s + cb - cur;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kBlock) tet_h_update(DevPtrs d) {
   __shared__ double sh[33];
+  cudaTriggerProgrammaticLaunchCompletion();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   double fl = 0.0;
-  if (e < d.nE && d.h_ptr[e + 1] > d.h_ptr[e]) {
-    const T* cf = (const T*)d.cf;
-    T s = 0;
-    for (int64_t k = d.h_ptr[e]; k < d.h_ptr[e + 1]; k++) s += ld<T>(d.h_val, k) * cf[d.h_col[k]];
+  const bool ok = e < d.nE && d.edge_upd[e];
+  T s = 0;
+  if (ok) s = tet_row<T, 9>(d.H, e, (const T*)d.cf, [] { cudaGridDependencySynchronize(); });
+  else cudaGridDependencySynchronize();
+  if (ok) {
     T* U = (T*)d.U;
     const T uo = U[e];
     const T un = d.h_p ? ((const T*)d.h_p)[e] * uo + (T)d.dt * s : uo + (T)d.dt * s;
@@ -110,8 +188,79 @@ __global__ void __launch_bounds__(kBlock) tet_h_update(DevPtrs d) {
     const T cb = ((const T*)d.cb)[e];
     if (cb != (T)0) fl = ((double)uo + (double)un) * (double)cb;
   }
-  fl = block_sum(fl, sh);
+  if (__syncthreads_or(fl != 0.0)) fl = block_sum(fl, sh);
   if (threadIdx.x == 0) d.flux_part[blockIdx.x] = fl;
+}
+
+// the last block sums the step's boundary flux
+template <typename T>
+__global__ void __launch_bounds__(kBlock) tet_curl_u(DevPtrs d) {
+  __shared__ double sh[33];
+  cudaTriggerProgrammaticLaunchCompletion();
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  int32_t e0 = 0, e1 = 0, e2 = 0;
+  if (f < d.nF) {
+    e0 = d.fte[f];
+    e1 = d.fte[d.nF + f];
+    e2 = d.fte[2 * (int64_t)d.nF + f];
+  }
+  cudaGridDependencySynchronize();
+  if (blockIdx.x == gridDim.x - 1) {
+    double a = 0.0;
+    for (int b = threadIdx.x; b < d.nflux_part; b += blockDim.x) a += d.flux_part[b];
+    a = block_sum(a, sh);
+    if (threadIdx.x == 0) {
+      d.flux[d.step[0]] = 0.5 * a;
+      d.step[1] = d.step[0];
+    }
+    return;
+  }
+  if (f >= d.nF) return;
+  const T* U = (const T*)d.U;
+  const T c = U[e0] - U[e1] + U[e2];
+  ((T*)d.cu)[f] = c;
+  T* B = (T*)d.B;
+  B[f] = B[f] - (T)d.dt * c;
+}
+
+// Probe export of component c (E x y z, H x y z) of probe p into print slot `slot`.
+template <typename T>
+__device__ __forceinline__ void tet_probe(const DevPtrs& d, int p, int c, int slot) {
+  const int a = c % 3;
+  double v = 0.0;
+  if (c < 3) {
+    const T* U = (const T*)d.U;
+    for (int q = 0; q < 6; q++) v += d.p_we[18 * (int64_t)p + 3 * q + a] * (double)U[d.p_edges[6 * (int64_t)p + q]];
+  } else {
+    const T* B = (const T*)d.B;
+    for (int q = 0; q < 4; q++) v += d.p_hf[12 * (int64_t)p + 3 * q + a] * (double)B[d.p_faces[4 * (int64_t)p + q]];
+  }
+  d.samples[((int64_t)slot * d.np + p) * 6 + c] = v;
+}
+
+// F = R F - dt N cu; the first npb blocks sample the probes, one thread per
+// probe and component, and advance the step counter
+template <typename T>
+__global__ void __launch_bounds__(kBlock) tet_nmul(DevPtrs d, int npb) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  if ((int)blockIdx.x < npb) {
+    cudaGridDependencySynchronize();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int step = d.step[1];  // tet_curl_u's copy: step[0] advances below
+    if (t == 0) d.step[0] = step + 1;
+    if (t >= 6 * d.np) return;
+    const int slot = d.slot_of_step[step + 1];
+    if (slot >= 0) tet_probe<T>(d, t / 6, t % 6, slot);
+    return;
+  }
+  const int f = (blockIdx.x - npb) * blockDim.x + threadIdx.x;
+  if (f >= d.nF) {
+    cudaGridDependencySynchronize();
+    return;
+  }
+  const T s = tet_row<T, 7>(d.N, f, (const T*)d.cu, [] { cudaGridDependencySynchronize(); });
+  T* F = (T*)d.F;
+  F[f] = d.n_r ? ((const T*)d.n_r)[f] * F[f] - (T)d.dt * s : F[f] - (T)d.dt * s;
 }
 
 template <typename T>
@@ -184,8 +333,9 @@ __global__ void __launch_bounds__(kBlock) tet_energy_m(DevPtrs d, double* part) 
   double c = 0.0;
   if (f < d.nF) {
     const T* B = (const T*)d.B;
+    const int64_t b = d.N.ptr[f >> 5] + (f & 31), e = d.N.ptr[(f >> 5) + 1];
     double s = 0.0;
-    for (int64_t k = d.n_ptr[f]; k < d.n_ptr[f + 1]; k++) s += (double)ld<T>(d.n_val, k) * (double)B[d.n_col[k]];
+    for (int64_t k = b; k < e; k += 32) s += (double)((const T*)d.N.val)[k] * (double)B[d.N.col[k]];
     c = (double)B[f] * s;
   }
   c = block_sum(c, sh);
@@ -201,44 +351,6 @@ __global__ void tet_energy_sum(const double* pe, int nbe, const double* pm, int 
   }
   for (int q = 0; q < nbm; q++) c += pm[q];
   *out = 0.5 * a + 0.5 * dt * b + 0.5 * c;
-}
-
-// Source edges: E sources write U, H sources write cb (reset each step),
-// currents write I.
-template <typename T>
-__global__ void __launch_bounds__(kBlock) tet_sources(DevPtrs d) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  const int step = *d.step;
-  if (s < d.nse) {
-    auto value = [&](int row) {
-      double v[3] = {0.0, 0.0, 0.0};
-      for (int p = d.se_begin[s]; p < d.se_begin[s + 1]; p++) {
-        const int si = d.pair_src[p];
-        double ret = d.src_amp[si] * d.carrier[(int64_t)row * d.nsrc + si];
-        ret *= d.pair_fac[4 * p + 0];
-        ret *= d.pair_fac[4 * p + 1];
-        ret *= d.pair_fac[4 * p + 2];
-        ret *= d.pair_fac[4 * p + 3];
-        v[d.pair_dir[p]] += ret;
-      }
-      const double* w = d.se_vec + 3 * (int64_t)s;
-      return d.se_post[s] * ((v[0] * w[0] + v[1] * w[1]) + v[2] * w[2]);
-    };
-    const int e = d.se_edge[s];
-    const int kind = d.se_kind[s];
-    const double val = value(step);
-    if (kind == 1) ((T*)d.U)[e] = (T)val;
-    else if (kind == 2) ((T*)d.cb)[e] = (T)val;
-    else if (kind == 3) ((T*)d.I)[e] = (T)val;
-  }
-}
-
-__global__ void flux_reduce(DevPtrs d, double scale) {
-  __shared__ double sh[33];
-  double a = 0.0;
-  for (int b = threadIdx.x; b < d.nflux_part; b += blockDim.x) a += d.flux_part[b];
-  a = block_sum(a, sh);
-  if (threadIdx.x == 0) d.flux[*d.step] = scale * a;
 }
 
 template <typename T>
@@ -355,34 +467,13 @@ __global__ void __launch_bounds__(kBlock) tet_cg(DevPtrs d) {
   }
 }
 
-// Probe export.  The print schedule is indexed by step counter + offset:
-// after a step, time (s+1) dt, offset 1; before the first step, offset 0.
+// export before the first step (t = 0)
 template <typename T>
-__global__ void tet_probes(DevPtrs d, int offset) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int step = *d.step;
-  const int slot = d.slot_of_step[step + offset];
-  if (p < d.np && slot >= 0) {
-    const T* U = (const T*)d.U;
-    const T* B = (const T*)d.B;
-    double E[3] = {0, 0, 0}, H[3] = {0, 0, 0};
-    for (int q = 0; q < 6; q++) {
-      const double u = (double)U[d.p_edges[6 * p + q]];
-      for (int a = 0; a < 3; a++) E[a] += d.p_we[18 * p + 3 * q + a] * u;
-    }
-    for (int q = 0; q < 4; q++) {
-      const double b = (double)B[d.p_faces[4 * p + q]];
-      for (int a = 0; a < 3; a++) H[a] += d.p_hf[12 * p + 3 * q + a] * b;
-    }
-    double* out = d.samples + ((int64_t)slot * d.np + p) * 6;
-    for (int a = 0; a < 3; a++) {
-      out[a] = E[a];
-      out[3 + a] = H[a];
-    }
-  }
+__global__ void __launch_bounds__(kBlock) tet_initial_probes(DevPtrs d) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int slot = d.slot_of_step[0];
+  if (t < 6 * d.np && slot >= 0) tet_probe<T>(d, t / 6, t % 6, slot);
 }
-
-__global__ void bump_step(int* step) { *step += 1; }
 
 // ------------------------------------------------------------------ launch
 static inline unsigned nblk(int64_t n) { return (unsigned)((n + kBlock - 1) / kBlock > 0 ? (n + kBlock - 1) / kBlock : 1); }
@@ -396,31 +487,54 @@ int tet_cg_blocks(int device) {
   return per_sm * sms;
 }
 
+// out[i] = v[where[i]]: a field in the reference's numbering, as double
+template <typename T>
+__global__ void __launch_bounds__(kBlock) tet_export(const T* v, const int32_t* where, double* out, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (double)v[where[i]];
+}
+template <typename T>
+cudaError_t tet_launch_export(const void* v, const int32_t* where, double* out, int n, cudaStream_t st) {
+  tet_export<T><<<nblk(n), kBlock, 0, st>>>((const T*)v, where, out, n);
+  return cudaGetLastError();
+}
+template cudaError_t tet_launch_export<double>(const void*, const int32_t*, double*, int, cudaStream_t);
+template cudaError_t tet_launch_export<float>(const void*, const int32_t*, double*, int, cudaStream_t);
+
 // One leapfrog step of the dga method (Discretization.hpp:810-931).  ev
-// (optional, 6 events) brackets: sources, H half, flux, E half, probes.
+// (optional, 6 events) brackets: sources (none of their own), H half, flux (in
+// the E half), E half, probes (in the E half).
 template <typename T>
 cudaError_t tet_launch_step(const DevPtrs& d, cudaStream_t st, cudaEvent_t* ev) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kBlock);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   if (ev) cudaEventRecord(ev[0], st);
-  cudaMemsetAsync(d.cb, 0, sizeof(T) * (size_t)d.nE, st);
-  if (d.nse) tet_sources<T><<<nblk(d.nse), kBlock, 0, st>>>(d);
   if (ev) cudaEventRecord(ev[1], st);
-  tet_curl_f<T><<<nblk(d.nE), kBlock, 0, st>>>(d);
-  tet_h_update<T><<<nblk(d.nE), kBlock, 0, st>>>(d);
+  cfg.gridDim = dim3(nblk(d.nE));
+  cudaError_t e = cudaLaunchKernelEx(&cfg, tet_curl_f<T, true>, d);
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, tet_h_update<T>, d);
+  if (e != cudaSuccess) return e;
   if (d.nq > 0) {
     cudaMemcpyAsync(d.Uc_old, d.Uc, sizeof(T) * (size_t)d.nq, cudaMemcpyDeviceToDevice, st);
     tet_frac_update<T><<<nblk(d.nq), kBlock, 0, st>>>(d);
   }
   if (d.nfe > 0) tet_frac_gather<T><<<nblk(d.nfe), kBlock, 0, st>>>(d, (int)nblk(d.nE));
   if (ev) cudaEventRecord(ev[2], st);
-  flux_reduce<<<1, kBlock, 0, st>>>(d, 0.5);
   if (ev) cudaEventRecord(ev[3], st);
-  tet_curl_u<T><<<nblk(d.nF), kBlock, 0, st>>>(d);
-  tet_nmul<T><<<nblk(d.nF), kBlock, 0, st>>>(d);
+  cfg.gridDim = dim3(nblk(d.nF) + 1);
+  e = cudaLaunchKernelEx(&cfg, tet_curl_u<T>, d);
+  const int npb = (int)nblk(6 * (int64_t)d.np);
+  cfg.gridDim = dim3(nblk(d.nF) + npb);
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, tet_nmul<T>, d, npb);
   if (ev) cudaEventRecord(ev[4], st);
-  if (d.np) tet_probes<T><<<nblk(d.np), kBlock, 0, st>>>(d, 1);
-  bump_step<<<1, 1, 0, st>>>(d.step);
   if (ev) cudaEventRecord(ev[5], st);
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // Jacobi preconditioner from the CSR diagonal (1 where the diagonal is
@@ -447,10 +561,9 @@ cudaError_t pcg_launch_solve(DevPtrs d, int blocks, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// export before the first step (dga: t = 0)
 template <typename T>
 void tet_launch_initial_probes(const DevPtrs& d, cudaStream_t st) {
-  if (d.np) tet_probes<T><<<nblk(d.np), kBlock, 0, st>>>(d, 0);
+  if (d.np) tet_initial_probes<T><<<nblk(6 * (int64_t)d.np), kBlock, 0, st>>>(d);
 }
 
 // dga energy: gather u, solve H x = u (d_cg: the class-1 block of H and the
@@ -458,7 +571,7 @@ void tet_launch_initial_probes(const DevPtrs& d, cudaStream_t st) {
 template <typename T>
 cudaError_t tet_launch_energy(const DevPtrs& d, DevPtrs d_cg, int cg_blocks, const int32_t* ie, int ni,
                               double* part, double* out, cudaStream_t st) {
-  tet_curl_f<T><<<nblk(d.nE), kBlock, 0, st>>>(d);
+  tet_curl_f<T, false><<<nblk(d.nE), kBlock, 0, st>>>(d);
   tet_energy_gather<T><<<nblk(ni), kBlock, 0, st>>>(d, ie, (double*)d_cg.rhs, ni);
   cudaMemsetAsync(d_cg.x, 0, sizeof(double) * (size_t)ni, st);
   cudaError_t e = pcg_launch_solve(d_cg, cg_blocks, st);

@@ -1,16 +1,26 @@
 // Device layout of the explicit tetrahedral DGA method (dga) and of the
 // standalone CG solve.
 //
+// The dga device numbering of edges and faces follows the form of their H and
+// N rows (TetSim::alloc_and_upload); states are exchanged in the reference's.
 // Complex: faces carry their three edges (p0p1, p0p2, p1p2 with signs +, -, +,
-// the reference's fte order, Discretization.hpp:6327-6352); C^T is a CSR over
-// edges whose int32 entries hold the face index with the sign in bit 31.  The
-// material operators are CSR with int32 columns: N (faces x faces, per-tet
-// inverse blocks summed) and H (masked node-star inverses); the CG solve takes
-// the caller's CSR system A.
+// the reference's fte order, Discretization.hpp:6327-6352), one array each;
+// C^T has int32 entries with the face and the sign in bit 31.  C^T, N (faces x
+// faces, per-tet inverse blocks summed) and H (masked node-star inverses) are
+// SELL-32 with int32 columns; the CG solve takes the caller's CSR system A.
 #pragma once
 #include <cstdint>
 
 namespace tf {
+
+// 32-row slices: entry j of row i at ptr[i / 32] + 32 j + i % 32.  Padding
+// entries have value 0 and the row's first column (C^T: kNoFace).
+struct TetSell {
+  const int64_t* ptr = nullptr;
+  const int32_t* col = nullptr;
+  const void* val = nullptr;
+};
+constexpr int32_t kNoFace = 0x7fffffff;
 
 // Type-erased device pointers (T = float or double arrays are void*).  The
 // dga step uses the complex, N, H, the state and the sources; the standalone
@@ -21,13 +31,14 @@ struct DevPtrs {
   // state (T)
   void *U = nullptr, *F = nullptr, *B = nullptr, *cu = nullptr, *cf = nullptr, *I = nullptr, *cb = nullptr;
   // complex
-  const int32_t* fte = nullptr;
-  const int64_t* ct_ptr = nullptr;
-  const int32_t* ct_col = nullptr;
-  // operators (values T)
-  const int64_t *n_ptr = nullptr, *h_ptr = nullptr, *a_ptr = nullptr;
-  const int32_t *n_col = nullptr, *h_col = nullptr, *a_col = nullptr;
-  const void *n_val = nullptr, *h_val = nullptr, *a_val = nullptr;
+  const int32_t* fte = nullptr;       // [3][nF]
+  TetSell Ct, N, H;                   // values T
+  const uint8_t* edge_upd = nullptr;  // edges with an H row
+  const int32_t* edge_src = nullptr;  // source edge of an edge, or -1
+  // the CG solve's system
+  const int64_t* a_ptr = nullptr;
+  const int32_t* a_col = nullptr;
+  const void* a_val = nullptr;
   const void* jac = nullptr;
   // dga with conducting tets: P per edge (null when lossless), the node-star
   // fractions U_c (and their copy from the step before) with their operators
@@ -69,7 +80,7 @@ struct DevPtrs {
   const double *p_we = nullptr, *p_hf = nullptr;
   double* samples = nullptr;
   const int* slot_of_step = nullptr;
-  int* step = nullptr;
+  int* step = nullptr;  // [0] step being made, [1] its copy for the step's last launch
 };
 
 }  // namespace tf
