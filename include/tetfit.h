@@ -169,8 +169,10 @@ TF_API int tf_training_loss(tf_ctx* ctx, float* loss, size_t cap, size_t* n);
  * ||r||/||r0|| <= tol (criterion 0) or ||r|| <= tol ||b|| (criterion 1), at
  * most maxiter iterations, 0 meaning 100).  x holds the initial guess and
  * receives the solution.  Returns TF_E_SOLVER when the iteration limit is hit
- * first (x then holds the last iterate).  Allocates its work space (4 n + a
- * few hundred doubles) on the device for the duration of the call.  Errors are
+ * first (x then holds the last iterate).  Work space: the array of
+ * tf_pcg_solve_noalloc when the system fits it and no other call is using it,
+ * else an allocation on the device (4 n doubles and a few MB) for the duration
+ * of the call.  Errors are
  * reported through tf_last_error(NULL). */
 typedef struct tf_pcg_args {
   int32_t n;                 /* rows = columns                                  */
@@ -196,8 +198,8 @@ TF_API int tf_pcg_solve(const tf_pcg_args* args, int32_t* iters, double* rel_res
  * until the process exits, and larger n is rejected with TF_E_ARG.  The first
  * call on a device looks up the array's device address (once per device, that
  * device current); make that first call before any stream capture.  All calls
- * share the one array: calls that overlap on the GPU (other streams, other host
- * threads) race and must be serialised by the caller.  The address lookup is
+ * share the one array: a call that finds it in use by another host thread waits
+ * for that call's results.  The address lookup is
  * kept for the life of the process, so cudaDeviceReset (which reloads the
  * module) is not supported while the library is loaded.  Same arguments,
  * results and status codes as tf_pcg_solve. */

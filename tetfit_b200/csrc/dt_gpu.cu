@@ -21,7 +21,8 @@
 #include "tet_kernels.cuh"
 
 namespace tf {
-cudaError_t pcg_launch_solve(DevPtrs d, int blocks, cudaStream_t st);
+cudaError_t pcg_launch_solve(DevPtrs d, int blocks, int device, cudaStream_t st);
+size_t pcg_box_bytes(int device);
 template <typename T>
 int tet_cg_blocks(int device);
 
@@ -187,6 +188,7 @@ double gpu_lanczos_lambda(const DtProblem& p) {
       cg.cg_limit = (int32_t*)(tail + 3);
       cg.err = (int*)(tail + 4);
       cg.gbar = (unsigned int*)(tail + 5);
+      cg.box = (uint4*)vec((int64_t)(pcg_box_bytes(p.device) / sizeof(double)));
       cg.tol = 1e-12;
       cg.cg_maxiter = 1000;
       cg.cg_criterion = 1;
@@ -200,7 +202,7 @@ double gpu_lanczos_lambda(const DtProblem& p) {
       DevPtrs d = cg;
       d.rhs = (void*)in;
       d.x = out;
-      CU(pcg_launch_solve(d, cg_blocks, st));
+      CU(pcg_launch_solve(d, cg_blocks, p.device, st));
       int berr = 0;
       CU(cudaMemcpyAsync(&berr, d.err, sizeof(int), cudaMemcpyDeviceToHost, st));
       CU(cudaStreamSynchronize(st));

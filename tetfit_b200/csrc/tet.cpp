@@ -36,7 +36,7 @@ cudaError_t tet_launch_export(const void* v, const int32_t* where, double* out, 
 template <typename T>
 void tet_launch_initial_probes(const DevPtrs& d, cudaStream_t st);
 template <typename T>
-cudaError_t tet_launch_energy(const DevPtrs& d, DevPtrs d_cg, int cg_blocks, const int32_t* ie, int ni,
+cudaError_t tet_launch_energy(const DevPtrs& d, DevPtrs d_cg, int cg_blocks, int device, const int32_t* ie, int ni,
                               double* part, double* out, cudaStream_t st);
 template <typename T>
 int tet_cg_blocks(int device);
@@ -2272,8 +2272,8 @@ double TetSim::dga_energy() {
     en_part_ = (double*)dalloc(nparts * 8);
     en_out_ = (double*)dalloc(8);
   }
-  cudaError_t e = f32 ? tet_launch_energy<float>(dp_, en_cg_, en_blocks_, en_edges_, en_n_, en_part_, en_out_, stream_)
-                      : tet_launch_energy<double>(dp_, en_cg_, en_blocks_, en_edges_, en_n_, en_part_, en_out_, stream_);
+  cudaError_t e = f32 ? tet_launch_energy<float>(dp_, en_cg_, en_blocks_, opt_.device, en_edges_, en_n_, en_part_, en_out_, stream_)
+                      : tet_launch_energy<double>(dp_, en_cg_, en_blocks_, opt_.device, en_edges_, en_n_, en_part_, en_out_, stream_);
   CU(e);
   double w = 0;
   int berr = 0;

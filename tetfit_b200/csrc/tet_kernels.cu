@@ -20,8 +20,14 @@
 //                     axpys fused, FP64 reductions in a fixed order, a hard
 //                     iteration limit and three bounded grid barriers per
 //                     iteration
+//   pcg_resident      the same solve for systems of up to 8 rows a thread with
+//                     one block an SM: rows and matrix on chip, two exchanges
+//                     of partial sums per iteration (cg_resident.cuh)
 #include <cuda_runtime.h>
 
+#include <atomic>
+
+#include "cg_resident.cuh"
 #include "grid_barrier.cuh"
 #include "tet_kernels.cuh"
 
@@ -467,6 +473,154 @@ __global__ void __launch_bounds__(kBlock) tet_cg(DevPtrs d) {
   }
 }
 
+// tet_cg for systems that fit one block an SM, R rows a thread: x, r, p and the
+// Jacobi factor in registers, the rows' entries in shared memory as 32-row
+// slices (as many slices as fit; the rest is read from the CSR each time), the
+// pair (z, p) of a column gathered with one load, where p_j = z + beta p_{j-1}
+// is formed with the rounding of the row's owner.  zp (2 n doubles) takes the
+// place of jac and r.  Bound by latency: 131 k rows of 7 entries took 22.8 us an
+// iteration with tet_cg, the call's other costs included, and take 9.5.
+constexpr int kPcgThreads = 512;
+
+template <int R>
+__global__ void __launch_bounds__(kPcgThreads, 1) pcg_resident(DevPtrs d, int rows_per_block, int entries) {
+  constexpr int CH = 7;
+  extern __shared__ __align__(16) unsigned char pcg_raw[];
+  __shared__ CgShared sh;
+  __shared__ int width[R * kPcgThreads / 32 + 1];
+  double* sval = reinterpret_cast<double*>(pcg_raw);
+  int32_t* scol = reinterpret_cast<int32_t*>(sval + entries);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+  const int n = d.nfree, r0 = blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
+  CgExchange ex{d.box, (int)gridDim.x, 0, (int)gridDim.x, d.err, &sh, 1u};
+  const double* val = (const double*)d.a_val;
+  const double* b = (const double*)d.rhs;
+  double* x = (double*)d.x;
+  double2* zp = (double2*)d.jac;
+  // slot k of a warp: rows r0 + 32 (k W + warp) + lane
+  int64_t at[R];
+  int len[R], off[R];
+  if (threadIdx.x == 0) sh.dead = 0;
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int i = r0 + 32 * (k * W + warp) + lane;
+    at[k] = i < r1 ? d.a_ptr[i] : 0;
+    len[k] = i < r1 ? (int)(d.a_ptr[i + 1] - at[k]) : 0;
+    const int w = __reduce_max_sync(0xffffffffu, len[k]);
+    if (lane == 0) width[k * W + warp] = w;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int s = 0;
+    for (int q = 0; q < R * W; q++) {
+      const int w = width[q];
+      width[q] = s + 32 * w <= entries ? s : -1;  // a slice that does not fit is read from the CSR
+      if (width[q] >= 0) s += 32 * w;
+    }
+  }
+  __syncthreads();
+  double xk[R], rk[R], pk[R], dk[R], qk[R];
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int i = r0 + 32 * (k * W + warp) + lane;
+    off[k] = width[k * W + warp];
+    double dg = 0.0;
+    if (off[k] >= 0) off[k] += lane;
+    for (int j = 0; j < len[k]; j++) {
+      const int32_t c = d.a_col[at[k] + j];
+      const double v = val[at[k] + j];
+      if (c == i) dg = v;
+      if (off[k] >= 0) {
+        scol[off[k] + 32 * j] = c;
+        sval[off[k] + 32 * j] = v;
+      }
+    }
+    dk[k] = dg != 0.0 ? 1.0 / dg : 1.0;
+    xk[k] = i < r1 ? x[i] : 0.0;
+    rk[k] = i < r1 ? b[i] : 0.0;
+    pk[k] = 0.0;
+    qk[k] = 0.0;
+  }
+  // a thread reads back the entries it wrote itself
+  auto row_dot = [&](int k, auto load, auto form) -> double {
+    double s = 0.0;
+    if (off[k] >= 0) {
+      for (int j0 = 0; j0 < len[k]; j0 += CH) {
+        decltype(load(0)) g[CH];
+#pragma unroll
+        for (int q = 0; q < CH; q++)
+          if (j0 + q < len[k]) g[q] = load(scol[off[k] + 32 * (j0 + q)]);
+#pragma unroll
+        for (int q = 0; q < CH; q++)
+          if (j0 + q < len[k]) s += sval[off[k] + 32 * (j0 + q)] * form(g[q]);
+      }
+    } else {
+      for (int j = 0; j < len[k]; j++) s += val[at[k] + j] * form(load(d.a_col[at[k] + j]));
+    }
+    return s;
+  };
+  double v3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int i = r0 + 32 * (k * W + warp) + lane;
+    if (i >= r1) continue;
+    const double bi = rk[k];
+    const double ri = bi - row_dot(k, [&](int32_t c) { return x[c]; }, [](double g) { return g; });
+    const double zi = __dmul_rn(dk[k], ri);
+    rk[k] = ri;
+    zp[i] = make_double2(zi, 0.0);
+    v3[0] += ri * ri;
+    v3[1] += ri * zi;
+    v3[2] += bi * bi;
+  }
+  bool alive = ex.sum<3, true>(v3);
+  const double res0 = sqrt(v3[0]), bnorm = sqrt(v3[2]);
+  double res = res0, rz = v3[1], beta = 0.0;
+  int it = 0;
+  auto unmet = [&]() { return d.cg_criterion == 0 ? res / res0 > d.tol : res > d.tol * bnorm; };  // NaN (res0 = 0) stops
+  while (alive && it < d.cg_maxiter && unmet()) {
+    const bool first = it == 0;
+    auto p_of = [&](double z, double p) { return first ? z : __fma_rn(beta, p, z); };
+    double v1[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      if (r0 + 32 * (k * W + warp) + lane >= r1) continue;
+      qk[k] = row_dot(k, [&](int32_t c) { return zp[c]; }, [&](double2 g) { return p_of(g.x, g.y); });
+      pk[k] = p_of(__dmul_rn(dk[k], rk[k]), pk[k]);
+      v1[0] += pk[k] * qk[k];
+    }
+    alive = ex.sum<1, false>(v1);
+    const double alpha = rz / v1[0];
+    double v2[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      const int i = r0 + 32 * (k * W + warp) + lane;
+      if (i >= r1) continue;
+      xk[k] = __fma_rn(alpha, pk[k], xk[k]);
+      rk[k] = rk[k] - alpha * qk[k];
+      const double zi = __dmul_rn(dk[k], rk[k]);
+      zp[i] = make_double2(zi, pk[k]);
+      v2[0] += rk[k] * rk[k];
+      v2[1] += rk[k] * zi;
+    }
+    alive = ex.sum<2, true>(v2) && alive;
+    res = sqrt(v2[0]);
+    beta = v2[1] / rz;
+    rz = v2[1];
+    it++;
+  }
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int i = r0 + 32 * (k * W + warp) + lane;
+    if (i < r1) x[i] = xk[k];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    d.cg_iters[0] = it;
+    d.cg_resid[0] = res / res0;
+    if (d.cg_limit) d.cg_limit[0] = unmet() ? 1 : 0;
+  }
+}
+
 // export before the first step (t = 0)
 template <typename T>
 __global__ void __launch_bounds__(kBlock) tet_initial_probes(DevPtrs d) {
@@ -548,13 +702,86 @@ __global__ void jacobi_from_csr(const int64_t* ptr, const int32_t* col, const do
   pre[i] = dg != 0.0 ? 1.0 / dg : 1.0;
 }
 
-// Standalone FP64 solve: preconditioner, then the persistent PCG kernel.
-cudaError_t pcg_launch_solve(DevPtrs d, int blocks, cudaStream_t st) {
+// Matrix entries a block's shared memory holds on a device, 0 when the kernel
+// cannot be launched; the limit the runtime has to be told is set on the first
+// call for the device (the set-up's estimate launches hundreds of solves).
+template <int R>
+static int pcg_resident_entries(int device) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices];
+  const bool keep = device >= 0 && device < kDevices;
+  if (keep && known[device].load() > 0) return known[device].load();
+  int most = 0, per_sm = 0;
+  cudaFuncAttributes fa{};
+  if (cudaFuncGetAttributes(&fa, pcg_resident<R>) != cudaSuccess ||
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+    return 0;
+  const int entries = (most - (int)fa.sharedSizeBytes) / (12 * 32) * 32;
+  if (cudaFuncSetAttribute(pcg_resident<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, entries * 12) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_resident<R>, kPcgThreads, entries * 12) != cudaSuccess ||
+      per_sm < 1)
+    return 0;
+  if (keep) known[device].store(entries);
+  return entries;
+}
+static int pcg_sms(int device) {
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return sms < 32 * kCgChunks ? sms : 32 * kCgChunks;
+}
+// bytes of DevPtrs::box
+size_t pcg_box_bytes(int device) {
+  const size_t g = (size_t)pcg_sms(device);
+  return 2 * kCgVals * g * g * sizeof(uint4);
+}
+
+// whether pcg_launch_solve takes the resident kernel (given boxes)
+bool pcg_resident_fits(int64_t n, int device) { return n <= (int64_t)8 * pcg_sms(device) * kPcgThreads; }
+
+template <int R>
+static cudaError_t pcg_launch_resident(const DevPtrs& d, int device, int sms, cudaStream_t st) {
+  const int entries = pcg_resident_entries<R>(device);
+  if (entries < 1) return cudaErrorLaunchOutOfResources;
+  // as few warps as one block an SM allows, but not fewer than 8
+  const int slices = (d.nfree + 31) / 32;
+  int W = (slices + sms * R - 1) / (sms * R);
+  W = W < 8 ? 8 : W;
+  int rows = 32 * W * R;
+  const int blocks = (d.nfree + rows - 1) / rows;
+  rows = ((slices + blocks - 1) / blocks) * 32;  // evenly
+  cudaMemsetAsync(d.box, 0, 2 * kCgVals * (size_t)blocks * blocks * sizeof(uint4), st);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((d.nfree + rows - 1) / rows);
+  cfg.blockDim = dim3(32 * W);
+  cfg.dynamicSmemBytes = (size_t)entries * 12;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, pcg_resident<R>, d, rows, entries);
+}
+
+// Standalone FP64 solve.  With boxes (DevPtrs::box) and at most 8 rows a thread
+// the resident kernel, which beat tet_cg at every size it takes (rows of 7
+// entries, us an iteration of a call: 1 k rows 5.3 against 21.1, 131 k 9.5
+// against 22.8, 594 k 31.8 against 35.8); otherwise preconditioner, then the
+// persistent PCG kernel.
+cudaError_t pcg_launch_solve(DevPtrs d, int blocks, int device, cudaStream_t st) {
+  cudaMemsetAsync(d.err, 0, sizeof(int), st);
+  if (d.box && pcg_resident_fits(d.nfree, device)) {
+    const int sms = pcg_sms(device);
+    const int64_t per = (int64_t)sms * kPcgThreads;  // rows of one row a thread
+    if (d.nfree <= per) return pcg_launch_resident<1>(d, device, sms, st);
+    if (d.nfree <= 2 * per) return pcg_launch_resident<2>(d, device, sms, st);
+    if (d.nfree <= 4 * per) return pcg_launch_resident<4>(d, device, sms, st);
+    return pcg_launch_resident<8>(d, device, sms, st);
+  }
   jacobi_from_csr<<<nblk(d.nfree), kBlock, 0, st>>>(d.a_ptr, d.a_col, (const double*)d.a_val, (double*)d.jac,
                                                     d.nfree);
   cudaMemsetAsync(d.step, 0, sizeof(int), st);
   cudaMemsetAsync(d.gbar, 0, 2 * sizeof(unsigned int), st);
-  cudaMemsetAsync(d.err, 0, sizeof(int), st);
   void* args[] = {(void*)&d};
   cudaError_t err = cudaLaunchCooperativeKernel((void*)tet_cg<double>, dim3(blocks), dim3(kBlock), args, 0, st);
   if (err != cudaSuccess) return err;
@@ -569,12 +796,12 @@ void tet_launch_initial_probes(const DevPtrs& d, cudaStream_t st) {
 // dga energy: gather u, solve H x = u (d_cg: the class-1 block of H and the
 // PCG work), then the three sums; *out receives W (device)
 template <typename T>
-cudaError_t tet_launch_energy(const DevPtrs& d, DevPtrs d_cg, int cg_blocks, const int32_t* ie, int ni,
+cudaError_t tet_launch_energy(const DevPtrs& d, DevPtrs d_cg, int cg_blocks, int device, const int32_t* ie, int ni,
                               double* part, double* out, cudaStream_t st) {
   tet_curl_f<T, false><<<nblk(d.nE), kBlock, 0, st>>>(d);
   tet_energy_gather<T><<<nblk(ni), kBlock, 0, st>>>(d, ie, (double*)d_cg.rhs, ni);
   cudaMemsetAsync(d_cg.x, 0, sizeof(double) * (size_t)ni, st);
-  cudaError_t e = pcg_launch_solve(d_cg, cg_blocks, st);
+  cudaError_t e = pcg_launch_solve(d_cg, cg_blocks, device, st);
   if (e != cudaSuccess) return e;
   const int nbe = (int)nblk(ni), nbm = (int)nblk(d.nF);
   tet_energy_e<T><<<nbe, kBlock, 0, st>>>(d, ie, (const double*)d_cg.x, ni, part);
@@ -583,9 +810,9 @@ cudaError_t tet_launch_energy(const DevPtrs& d, DevPtrs d_cg, int cg_blocks, con
   return cudaGetLastError();
 }
 
-template cudaError_t tet_launch_energy<double>(const DevPtrs&, DevPtrs, int, const int32_t*, int, double*, double*,
+template cudaError_t tet_launch_energy<double>(const DevPtrs&, DevPtrs, int, int, const int32_t*, int, double*, double*,
                                                cudaStream_t);
-template cudaError_t tet_launch_energy<float>(const DevPtrs&, DevPtrs, int, const int32_t*, int, double*, double*,
+template cudaError_t tet_launch_energy<float>(const DevPtrs&, DevPtrs, int, int, const int32_t*, int, double*, double*,
                                               cudaStream_t);
 template cudaError_t tet_launch_step<double>(const DevPtrs&, cudaStream_t, cudaEvent_t*);
 template cudaError_t tet_launch_step<float>(const DevPtrs&, cudaStream_t, cudaEvent_t*);

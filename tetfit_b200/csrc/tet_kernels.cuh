@@ -9,6 +9,8 @@
 // faces, per-tet inverse blocks summed) and H (masked node-star inverses) are
 // SELL-32 with int32 columns; the CG solve takes the caller's CSR system A.
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace tf {
@@ -56,7 +58,9 @@ struct DevPtrs {
   void *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *rhs = nullptr;
   double *part_a = nullptr, *part_b = nullptr;
   unsigned int* gbar = nullptr;  // grid barrier: arrivals, generation
-  int* err = nullptr;            // raised when a grid barrier wait ran out of time
+  int* err = nullptr;            // raised when a wait of the solve ran out of time
+  uint4* box = nullptr;          // optional: exchange boxes of the resident solve (pcg_box_bytes); with them jac
+                                 // has room for 2 nfree doubles, 16-byte aligned
   int32_t* cg_iters = nullptr;
   double* cg_resid = nullptr;
   int32_t* cg_limit = nullptr;  // optional: 1 when the iteration limit stopped the solve
