@@ -633,8 +633,21 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
   SimCg* st = reinterpret_cast<SimCg*>(smem_raw);
   auto grid_sync = [&]() { grid_barrier(d.gbar, d.err, gridDim.x); };
   double* wp = reinterpret_cast<double*>(smem_raw + sizeof(SimCg) * d.S);
+  // the block's segments: first and last slice, simulation, number (looked up
+  // in global memory for every segment and phase, two dependent loads, they
+  // cost a batch of 16 members a third of its solve)
+  __shared__ int64_t seg_a[kMaxSeg], seg_b[kMaxSeg];
+  __shared__ int seg_s[kMaxSeg], seg_g[kMaxSeg];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g0 = d.blk_seg[blockIdx.x], g1 = d.blk_seg[blockIdx.x + 1];
+  const int ng = d.blk_seg[blockIdx.x + 1] - d.blk_seg[blockIdx.x];
+  if (threadIdx.x < ng) {
+    const int g = d.seg_of[d.blk_seg[blockIdx.x] + threadIdx.x];
+    seg_g[threadIdx.x] = g;
+    seg_s[threadIdx.x] = d.seg_sim[g];
+    seg_a[threadIdx.x] = d.seg_s0[g];
+    seg_b[threadIdx.x] = d.seg_s1[g];
+  }
+  __syncthreads();
   T* x = (T*)d.x;
   T* r = (T*)d.r;
   T* q = (T*)d.q;
@@ -651,7 +664,7 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
     a3 = warp_sum(a3);
     a4 = warp_sum(a4);
     if (lane == 0) {
-      double* w = wp + ((g - g0) * cg_warps<T>() + warp) * kPart;
+      double* w = wp + (g * cg_warps<T>() + warp) * kPart;
       w[3] = a3;
       w[4] = a4;
     }
@@ -659,31 +672,34 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
     a1 = warp_sum(a1);
     a2 = warp_sum(a2);
     if (lane == 0) {
-      double* w = wp + ((g - g0) * cg_warps<T>() + warp) * kPart;
+      double* w = wp + (g * cg_warps<T>() + warp) * kPart;
       w[0] = a0;
       w[1] = a1;
       w[2] = a2;
     }
   };
-  auto flush = [&](int g, double a0, double a1, double a2) {
+  auto flush1 = [&](int g, double a0) {
+    a0 = warp_sum(a0);
+    if (lane == 0) wp[(g * cg_warps<T>() + warp) * kPart] = a0;
+  };
+  auto flush2 = [&](int g, double a0, double a1) {
     a0 = warp_sum(a0);
     a1 = warp_sum(a1);
-    a2 = warp_sum(a2);
     if (lane == 0) {
-      double* w = wp + ((g - g0) * cg_warps<T>() + warp) * kPart;
+      double* w = wp + (g * cg_warps<T>() + warp) * kPart;
       w[0] = a0;
       w[1] = a1;
-      w[2] = a2;
     }
   };
+  // the block's sums of each segment: one warp per segment and value, lanes
+  // over the warps, a fixed shuffle tree
   auto publish = [&](int nq, int slot) {
     __syncthreads();
-    for (int gl = threadIdx.x; gl < g1 - g0; gl += cg_threads<T>())
-      for (int k = 0; k < nq; k++) {
-        double a = 0.0;
-        for (int w = 0; w < cg_warps<T>(); w++) a += wp[(gl * cg_warps<T>() + w) * kPart + k];
-        d.part[kCgPart * (int64_t)d.seg_of[g0 + gl] + slot + k] = a;
-      }
+    for (int t = warp; t < ng * nq; t += cg_warps<T>()) {
+      const int g = t / nq, k = t - g * nq;
+      const double a = warp_sum(lane < cg_warps<T>() ? wp[(g * cg_warps<T>() + lane) * kPart + k] : 0.0);
+      if (lane == 0) d.part[kCgPart * (int64_t)seg_g[g] + slot + k] = a;
+    }
   };
   // per-simulation totals of the published partials: one warp per
   // simulation, lanes over its segments, then a fixed shuffle tree; f(s, t)
@@ -708,11 +724,11 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
   T* ra = (T*)d.r_alt;
   T* za = (T*)d.z_alt;
   const bool dual = d.dual != 0;
-  for (int g = g0; g < g1; g++) {
-    const int s = d.seg_sim[d.seg_of[g]];
+  for (int g = 0; g < ng; g++) {
+    const int s = seg_s[g];
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0, a4 = 0.0;
     if (running(d, s))
-      for (int64_t sl = d.seg_s0[d.seg_of[g]] + warp; sl < d.seg_s1[d.seg_of[g]]; sl += cg_warps<T>()) {
+      for (int64_t sl = seg_a[g] + warp; sl < seg_b[g]; sl += cg_warps<T>()) {
         const int64_t i = sl * 32 + lane;
         const T ri = b[i] - sell_dot_cg<T>(d.A, i, [&](int32_t c) { return x[c]; });
         r[i] = ri;
@@ -756,8 +772,8 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
     if (!__syncthreads_or(any)) break;
     // p_{j+1} = z + beta p_j, x += alpha_j p_j (lazy), and in the fused
     // variant q = A p_{j+1} with p.q partials
-    for (int g = g0; g < g1; g++) {
-      const int s = d.seg_sim[d.seg_of[g]];
+    for (int g = 0; g < ng; g++) {
+      const int s = seg_s[g];
       const SimCg c = st[s];
       double a0 = 0.0;
       if (c.active) {
@@ -767,7 +783,7 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
         T* pn = pbuf(c.it);
         T* xs = xs_of(c);
         const T* zs = zs_of(c);
-        for (int64_t sl = d.seg_s0[d.seg_of[g]] + warp; sl < d.seg_s1[d.seg_of[g]]; sl += cg_warps<T>()) {
+        for (int64_t sl = seg_a[g] + warp; sl < seg_b[g]; sl += cg_warps<T>()) {
           const int64_t i = sl * 32 + lane;
           const T po = first ? (T)0 : pold[i];
           const T pi = p_next<T>(zs[i], po, beta, first);
@@ -782,24 +798,24 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
           }
         }
       }
-      if (kFused) flush(g, a0, 0.0, 0.0);
+      if (kFused) flush1(g, a0);
     }
     if (!kFused) {
       grid_sync();
-      for (int g = g0; g < g1; g++) {
-        const int s = d.seg_sim[d.seg_of[g]];
+      for (int g = 0; g < ng; g++) {
+        const int s = seg_s[g];
         const SimCg c = st[s];
         double a0 = 0.0;
         if (c.active) {
           const T* pn = pbuf(c.it);
-          for (int64_t sl = d.seg_s0[d.seg_of[g]] + warp; sl < d.seg_s1[d.seg_of[g]]; sl += cg_warps<T>()) {
+          for (int64_t sl = seg_a[g] + warp; sl < seg_b[g]; sl += cg_warps<T>()) {
             const int64_t i = sl * 32 + lane;
             const T qi = sell_dot_cg<T>(d.A, i, [&](int32_t cc) { return pn[cc]; });
             q[i] = qi;
             a0 += (double)pn[i] * (double)qi;
           }
         }
-        flush(g, a0, 0.0, 0.0);
+        flush1(g, a0);
       }
     }
     publish(1, kSlotPq);
@@ -809,14 +825,14 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
     });
     __syncthreads();
     // r -= alpha q; rr, rz partials
-    for (int g = g0; g < g1; g++) {
-      const int s = d.seg_sim[d.seg_of[g]];
+    for (int g = 0; g < ng; g++) {
+      const int s = seg_s[g];
       double a0 = 0.0, a1 = 0.0;
       if (st[s].active) {
         const T alpha = (T)st[s].alpha;
         T* rs = rs_of(st[s]);
         T* zs = zs_of(st[s]);
-        for (int64_t sl = d.seg_s0[d.seg_of[g]] + warp; sl < d.seg_s1[d.seg_of[g]]; sl += cg_warps<T>()) {
+        for (int64_t sl = seg_a[g] + warp; sl < seg_b[g]; sl += cg_warps<T>()) {
           const int64_t i = sl * 32 + lane;
           const T ri = rs[i] - alpha * q[i];
           rs[i] = ri;
@@ -827,7 +843,7 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
           a1 += rd * (double)zi;
         }
       }
-      flush(g, a0, a1, 0.0);
+      flush2(g, a0, a1);
     }
     publish(2, kSlotRes);
     grid_sync();
@@ -845,14 +861,14 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
     __syncthreads();
   }
   // the last x update, x += alpha_{J-1} p_{J-1}
-  for (int g = g0; g < g1; g++) {
-    const int s = d.seg_sim[d.seg_of[g]];
+  for (int g = 0; g < ng; g++) {
+    const int s = seg_s[g];
     const SimCg c = st[s];
     if (!running(d, s)) continue;
     const T alpha = (T)c.alpha;
     const T* pl = pbuf(c.it - 1);
     T* xs = xs_of(c);
-    for (int64_t sl = d.seg_s0[d.seg_of[g]] + warp; sl < d.seg_s1[d.seg_of[g]]; sl += cg_warps<T>()) {
+    for (int64_t sl = seg_a[g] + warp; sl < seg_b[g]; sl += cg_warps<T>()) {
       const int64_t i = sl * 32 + lane;
       T v = xs[i];
       if (c.it > 0) v = fmaT(alpha, pl[i], v);
