@@ -485,6 +485,20 @@ void TetGroup::build(std::vector<TetSim*>& sims, bool release_host) {
   }
   d.stat_off = (const int64_t*)upload(stat_off);
   d.sim_se = (const int*)upload(sim_se);
+  {
+    std::vector<int> sb_sim, sim_sb(S + 1, 0);
+    for (int q = 0; q < S; q++) {
+      const int nb = std::max(1, (sim_se[q + 1] - sim_se[q] + 255) / 256);  // kGB edges a block
+      sb_sim.insert(sb_sim.end(), nb, q);
+      sim_sb[q + 1] = sim_sb[q] + nb;
+    }
+    d.nsb = (int)sb_sim.size();
+    d.sb_sim = (const int*)upload(sb_sim);
+    d.sim_sb = (const int*)upload(sim_sb);
+    d.sb_flux = (double*)dalloc(sizeof(double) * sb_sim.size());
+    d.sb_count = (int*)dalloc(sizeof(int) * S);
+    CU(cudaMemset(d.sb_count, 0, sizeof(int) * S));
+  }
   d.se_edge = (const int32_t*)upload(se_edge);
   d.se_kind = (const int8_t*)upload(se_kind);
   d.se_begin = (const int*)upload(se_begin);

@@ -55,7 +55,7 @@ class TetGroup {
   double energy(int s);
   uint64_t device_bytes() const { return dev_bytes_; }
   int kernels_per_step() const {
-    return (cg_variant_ == kCgResident ? 6 : 7) + (dev_.np ? 1 : 0) + (opt_.warm_start == 3 ? 2 : 0) + (dev_.nsa ? 2 : 0);
+    return (cg_variant_ == kCgResident ? 6 : 7) + (opt_.warm_start == 3 ? 2 : 0) + (dev_.nsa ? 2 : 0);
   }
   int cg_blocks() const { return cg_blocks_; }
   int cg_variant() const { return cg_variant_; }

@@ -3,9 +3,9 @@
 //
 //   grp_curl_u     B -= dt C U on the faces (3 signed edges per face)
 //   grp_nmul       F = N B (SELL-32)
-//   grp_probes     Whitney E and face-flux H at the probe points (:3768-3897)
-//   grp_sources    one block per simulation: source-edge values from the
-//                  carrier table, boundary flux of the step (:1478-1504)
+//   grp_sources    source-edge values from the carrier table, boundary flux of
+//                  the step (:1478-1504); Whitney E and face-flux H at the
+//                  probe points (:3768-3897)
 //   grp_rhs        Psi = E (U_old - Src) - dt I + dt C^T F + dt Ctb Fb on the
 //                  free rows (:1516-1523) and the CG initial guess
 //   grp_cg         persistent cooperative Jacobi-PCG over every simulation's
@@ -241,39 +241,26 @@ __global__ void __launch_bounds__(kGB) grp_nmul(GroupDev d) {
   ((T*)d.F)[f] = sell_dot<T>(d.N, f, [&](int32_t c) { return B[c]; });
 }
 
-// gfdtd exports U^{i-1} and B^{i-1/2} inside step i (Discretization.hpp:1469-1475)
+// Component c (E x y z, H x y z) of probe p.  gfdtd exports U^{i-1} and B^{i-1/2}
+// inside step i (Discretization.hpp:1469-1475).
 template <typename T>
-__global__ void grp_probes(GroupDev d) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= d.np) return;
+__device__ __forceinline__ void grp_probe(const GroupDev& d, int64_t p, int c) {
   const int s = d.probe_sim[p];
   if (!running(d, s)) return;
   const int slot = d.sched[d.sched_off[s] + d.step[s]];
   if (slot < 0) return;
-  const T* U = (const T*)d.U;
-  const T* B = (const T*)d.B;
-  double E[3] = {0, 0, 0}, H[3] = {0, 0, 0};
-  for (int q = 0; q < 6; q++) {
-    const double u = (double)U[d.p_edges[6 * p + q]];
-    for (int a = 0; a < 3; a++) E[a] += d.p_we[18 * p + 3 * q + a] * u;
+  const int a = c % 3;
+  double v = 0.0;
+  if (c < 3) {
+    const T* U = (const T*)d.U;
+    for (int q = 0; q < 6; q++) v += d.p_we[18 * p + 3 * q + a] * (double)U[d.p_edges[6 * p + q]];
+  } else {
+    const T* B = (const T*)d.B;
+    for (int q = 0; q < 4; q++) v += d.p_hf[12 * p + 3 * q + a] * (double)B[d.p_faces[4 * p + q]];
   }
-  for (int q = 0; q < 4; q++) {
-    const double b = (double)B[d.p_faces[4 * p + q]];
-    for (int a = 0; a < 3; a++) H[a] += d.p_hf[12 * p + 3 * q + a] * b;
-  }
-  const int64_t nps = d.sim_probe[s + 1] - d.sim_probe[s];
-  double* out = d.samples + d.samp_off[s] + ((int64_t)slot * nps + (p - d.sim_probe[s])) * 6;
-  for (int a = 0; a < 3; a++) {
-    out[a] = E[a];
-    out[3 + a] = H[a];
-  }
-  if (d.io_out) {  // step_io: the same sample, contiguous per member
-    double* o2 = d.io_out + d.io_out_off[s] + (p - d.sim_probe[s]) * 6;
-    for (int a = 0; a < 3; a++) {
-      o2[a] = E[a];
-      o2[3 + a] = H[a];
-    }
-  }
+  const int64_t nps = d.sim_probe[s + 1] - d.sim_probe[s], k = p - d.sim_probe[s];
+  d.samples[d.samp_off[s] + ((int64_t)slot * nps + k) * 6 + c] = v;
+  if (d.io_out) d.io_out[d.io_out_off[s] + k * 6 + c] = v;  // step_io: the same sample, contiguous per member
 }
 
 __global__ void grp_io_carriers(GroupDev d, const double* in) {
@@ -290,20 +277,31 @@ cudaError_t group_launch_io_carriers(const GroupDev& d, const double* in, cudaSt
   return cudaGetLastError();
 }
 
-// One block per simulation.  E sources write the Dirichlet values, H sources
-// the boundary dual-edge term, currents I; the step's flux sum is
-// U_prev . 0.5 (Fb(t) + Fb(t - dt)) over the H-source edges.
+// Source edges, 256 a block (each block one simulation's), then the probes, one
+// thread per probe and component.  E sources write the Dirichlet values, H
+// sources the boundary dual-edge term, currents I; the step's flux sum is
+// U_prev . 0.5 (Fb(t) + Fb(t - dt)) over the H-source edges: the last block of a
+// simulation to arrive adds the blocks' sums in their order.  (With one block
+// a simulation, 40^3's 4,800 edges took 52 us.)
 template <typename T>
 __global__ void __launch_bounds__(kGB) grp_sources(GroupDev d) {
   __shared__ double sh[33];
-  const int s = blockIdx.x;
+  __shared__ bool last;
+  if ((int)blockIdx.x >= d.nsb) {
+    const int64_t t = (int64_t)((int)blockIdx.x - d.nsb) * kGB + threadIdx.x;
+    if (t < 6 * d.np) grp_probe<T>(d, t / 6, (int)(t % 6));
+    return;
+  }
+  const int s = d.sb_sim[blockIdx.x];
   if (!running(d, s)) return;
   const int step = d.step[s];
   const int ns = d.nsrc[s];
   const double* car = d.carrier + d.car_off[s];
   const int s0 = d.src_off[s];
+  const int b0 = d.sim_sb[s], b1 = d.sim_sb[s + 1];
+  const int k = d.sim_se[s] + ((int)blockIdx.x - b0) * kGB + threadIdx.x;
   double fl = 0.0;
-  for (int k = d.sim_se[s] + threadIdx.x; k < d.sim_se[s + 1]; k += kGB) {
+  if (k < d.sim_se[s + 1]) {
     auto value = [&](int row) {
       double v[3] = {0.0, 0.0, 0.0};
       for (int p = d.se_begin[k]; p < d.se_begin[k + 1]; p++) {
@@ -313,7 +311,10 @@ __global__ void __launch_bounds__(kGB) grp_sources(GroupDev d) {
         ret *= d.pair_fac[4 * p + 1];
         ret *= d.pair_fac[4 * p + 2];
         ret *= d.pair_fac[4 * p + 3];
-        v[d.pair_dir[p]] += ret;
+        const int a = d.pair_dir[p];
+        if (a == 0) v[0] += ret;
+        else if (a == 1) v[1] += ret;
+        else v[2] += ret;
       }
       const double* w = d.se_vec + 3 * (int64_t)k;
       return d.se_post[k] * ((v[0] * w[0] + v[1] * w[1]) + v[2] * w[2]);
@@ -327,13 +328,25 @@ __global__ void __launch_bounds__(kGB) grp_sources(GroupDev d) {
       const double prev = step > 0 ? value(step - 1) : 0.0;
       // gfdtd: Ctb Fb; fem: Ctb (Fb - Fb_old) (Discretization.hpp:1713)
       ((T*)d.cb)[e] = (T)(d.fem && d.fem[s] ? val - prev : val);
-      fl += (double)((const T*)d.U)[e] * (0.5 * (val + prev));
+      fl = (double)((const T*)d.U)[e] * (0.5 * (val + prev));
     } else if (kind == 3) {
       ((T*)d.I)[e] = (T)val;
     }
   }
   fl = grp_block_sum(fl, sh);
-  if (threadIdx.x == 0) d.flux[d.stat_off[s] + step] = fl;
+  if (threadIdx.x == 0) {
+    d.sb_flux[blockIdx.x] = fl;
+    __threadfence();
+    last = atomicAdd(&d.sb_count[s], 1) == b1 - b0 - 1;
+    if (last) d.sb_count[s] = 0;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double a = 0.0;
+  for (int q = b0 + (int)threadIdx.x; q < b1; q += kGB) a += *(volatile double*)&d.sb_flux[q];
+  a = grp_block_sum(a, sh);
+  if (threadIdx.x == 0) d.flux[d.stat_off[s] + step] = a;
 }
 
 // Right-hand side on the free rows and the initial guess: 0 previous
@@ -1315,7 +1328,7 @@ int group_guess_tc_blocks(int device) {
 }
 
 // One step of every running simulation.  ev (optional, 6 events) brackets:
-// H update + probes, sources + rhs, CG, scatter, step end.
+// H update, sources + probes + rhs, CG, scatter, step end.
 template <typename T>
 cudaError_t group_launch_step(const GroupDev& d, int cg_blocks, int cg_variant, size_t smem, cudaStream_t st,
                               cudaEvent_t* ev) {
@@ -1326,9 +1339,8 @@ cudaError_t group_launch_step(const GroupDev& d, int cg_blocks, int cg_variant, 
   }
   grp_curl_u<T><<<gblk(d.nF), kGB, 0, st>>>(d);
   grp_nmul<T><<<gblk(d.nF), kGB, 0, st>>>(d);
-  if (d.np) grp_probes<T><<<(unsigned)((d.np + 127) / 128), 128, 0, st>>>(d);
   if (ev) cudaEventRecord(ev[1], st);
-  grp_sources<T><<<d.S, kGB, 0, st>>>(d);
+  grp_sources<T><<<(unsigned)(d.nsb + (6 * d.np + kGB - 1) / kGB), kGB, 0, st>>>(d);
   grp_rhs<T><<<gblk(d.nrow), kGB, 0, st>>>(d);
   if (d.warm_start == 3) {
     grp_resid_e<T><<<gblk(d.nrow), kGB, 0, st>>>(d);

@@ -146,6 +146,13 @@ struct GroupDev {
   const int64_t* stat_off = nullptr;  // per simulation: first entry of its per-step arrays
   // sources (simulation s owns source edges [sim_se[s], sim_se[s+1]))
   const int* sim_se = nullptr;
+  // blocks of grp_sources: the simulation of each, the first block of each
+  // simulation [S + 1] (one at least), their flux sums and arrivals
+  int nsb = 0;
+  const int* sb_sim = nullptr;
+  const int* sim_sb = nullptr;
+  double* sb_flux = nullptr;
+  int* sb_count = nullptr;
   const int32_t* se_edge = nullptr;
   const int8_t* se_kind = nullptr;
   const int* se_begin = nullptr;
