@@ -22,8 +22,11 @@ namespace tf {
 constexpr int kCgVals = 5;     // most values of an exchange
 constexpr int kCgChunks = 10;  // 32-block chunks of a system
 
+constexpr int kCgCluster = 16;  // most blocks of a cluster
+
 struct CgShared {
   double warp[kCgVals][32];
+  double part[kCgVals][kCgCluster];  // of the cluster's blocks, in its first block
   double total[kCgVals * kCgChunks];
   int dead;
   alignas(8) uint64_t bar;  // the matrix copy's mbarrier
@@ -40,6 +43,11 @@ __device__ __forceinline__ double cg_warp_sum(double v) {
 // which keeps the pollers out of one another's way (148 blocks reading one set
 // of 148 records wait 3 to 5 us for one another in L2, with boxes 2 to 3).
 // box[parity][value][block][producer]
+//
+// With clusters of `cluster` blocks (one system a launch, at most 32 clusters)
+// a block hands its sums to the cluster's first block through distributed
+// shared memory, those exchange records with one another, and hand the totals
+// back: fewer records in flight, and none for a system of one cluster.
 struct CgExchange {
   uint4* box;
   int blocks;       // boxes per value, and records of a box
@@ -47,6 +55,87 @@ struct CgExchange {
   int* err;
   CgShared* sh;
   uint32_t round;   // number of the next exchange
+  int cluster;      // blocks of a cluster, 1 none
+
+  // Waits for the record of exchange k at p; false when it ran out.
+  template <bool kAcquire>
+  __device__ __forceinline__ bool read(const uint4* p, uint32_t k, double& a) {
+    uint64_t t0 = 0;
+    for (uint32_t n = 0;; n++) {
+      uint32_t x, fx, y, fy;
+      if (kAcquire)
+        asm volatile("ld.acquire.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(x), "=r"(fx), "=r"(y), "=r"(fy)
+                     : "l"(p)
+                     : "memory");
+      else
+        asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(x), "=r"(fx), "=r"(y), "=r"(fy)
+                     : "l"(p)
+                     : "memory");
+      if (fx == k && fy == k) {
+        a = __hiloint2double((int)y, (int)x);
+        return true;
+      }
+      if ((n & 255) == 255) {  // no clock read in a wait that ends at once
+        const uint64_t now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (*(volatile int*)err != 0 || now - t0 > kBarrierLimitNs) {
+          atomicOr(err, kBarrierTimedOut);
+          return false;
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void write(uint4* p, uint32_t k, double a) {
+    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"((uint32_t)__double2loint(a)),
+                 "r"(k), "r"((uint32_t)__double2hiint(a)), "r"(k)
+                 : "memory");
+  }
+  static __device__ __forceinline__ uint32_t peer(const void* p, int rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(a)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+  }
+  static __device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+
+  // sum() with clusters, from the warps' sums on
+  template <int NV, bool kPublish>
+  __device__ __forceinline__ void cluster_sum(uint32_t k) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+    const int rank = blockIdx.x % cluster, me = blockIdx.x / cluster, clusters = count / cluster;
+    for (int q = warp; q < NV; q += W) {
+      const double t = cg_warp_sum(lane < W ? sh->warp[q][lane] : 0.0);
+      if (lane == 0)
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer(&sh->part[q][rank], 0)), "d"(t) : "memory");
+    }
+    cluster_sync();
+    if (rank == 0)
+      for (int q = warp; q < NV; q += W) {
+        double t = __shfl_sync(0xffffffffu, cg_warp_sum(lane < cluster ? sh->part[q][lane] : 0.0), 0);
+        if (clusters > 1) {
+          uint4* set = box + ((size_t)(k & 1) * kCgVals + q) * blocks * blocks;
+          if (kPublish) __threadfence();
+          double a = 0.0;
+          if (lane < clusters) {
+            write(set + (size_t)lane * clusters + me, k, t);
+            if (!read<kPublish>(set + (size_t)me * clusters + lane, k, a)) sh->dead = 1;
+          }
+          t = __shfl_sync(0xffffffffu, cg_warp_sum(a), 0);
+          __syncwarp();
+        }
+        if (lane < cluster) {
+          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer(&sh->total[q], lane)), "d"(t) : "memory");
+          if (*(volatile int*)&sh->dead)
+            asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(peer(&sh->dead, lane)) : "memory");
+        }
+      }
+    cluster_sync();
+  }
 
   // v[] becomes the sums over the system's threads.  With kPublish, global
   // stores made before the call by any thread of the system are visible to
@@ -62,6 +151,12 @@ struct CgExchange {
 #pragma unroll
       for (int q = 0; q < NV; q++) sh->warp[q][warp] = v[q];
     __syncthreads();
+    if (cluster > 1) {
+      cluster_sum<NV, kPublish>(k);
+#pragma unroll
+      for (int q = 0; q < NV; q++) v[q] = sh->total[q];
+      return sh->dead == 0;
+    }
     // a warp adds the block's warps, writes to 32 boxes, then reads 32 records
     for (int t = warp; t < NV * chunks; t += W) {
       const int q = t / chunks, i = (t - q * chunks) * 32 + lane;
@@ -69,38 +164,8 @@ struct CgExchange {
       double a = __shfl_sync(0xffffffffu, cg_warp_sum(lane < W ? sh->warp[q][lane] : 0.0), 0);
       if (kPublish) __threadfence();
       if (i < count) {
-        asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(set + (size_t)(first + i) * blocks +
-                                                                                  me),
-                     "r"((uint32_t)__double2loint(a)), "r"(k), "r"((uint32_t)__double2hiint(a)), "r"(k)
-                     : "memory");
-        const uint4* p = set + (size_t)(first + me) * blocks + i;
-        uint64_t t0 = 0;
-        for (uint32_t n = 0;; n++) {
-          uint32_t x, fx, y, fy;
-          if (kPublish)
-            asm volatile("ld.acquire.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(x), "=r"(fx), "=r"(y), "=r"(fy)
-                         : "l"(p)
-                         : "memory");
-          else
-            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(x), "=r"(fx), "=r"(y), "=r"(fy)
-                         : "l"(p)
-                         : "memory");
-          if (fx == k && fy == k) {
-            a = __hiloint2double((int)y, (int)x);
-            break;
-          }
-          if ((n & 255) == 255) {  // no clock read in a wait that ends at once
-            const uint64_t now = global_ns();
-            if (t0 == 0) t0 = now;
-            if (*(volatile int*)err != 0 || now - t0 > kBarrierLimitNs) {
-              atomicOr(err, kBarrierTimedOut);
-              sh->dead = 1;
-              break;
-            }
-          }
-        }
+        write(set + (size_t)(first + i) * blocks + me, k, a);
+        if (!read<kPublish>(set + (size_t)(first + me) * blocks + i, k, a)) sh->dead = 1;
       } else {
         a = 0.0;
       }

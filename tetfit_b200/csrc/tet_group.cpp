@@ -713,8 +713,34 @@ bool TetGroup::resident() {
   if (R > kCgResidentRows) return false;
   int W = 8;
   while (W < kCgResidentWarps && blocks((int64_t)W * R) > sms) W++;
-  const int entries = group_resident_entries<T>(opt_.device, R);
+  int entries = group_resident_entries<T>(opt_.device, R);
   if (entries == 0) return false;
+  // Clusters (one simulation): one of 16 blocks when the rows fit it, a row a
+  // thread (9^3 FP64 141 -> 120 us a solve); as many of 8 as run at once, 15 on
+  // 148 SMs, when the exchange is between more than 80 blocks and the rows a
+  // thread are few (FP64: up to 2, 16^3 212 -> 184 us, 24^3 285 -> 244, with 3
+  // 27^3 293 -> 311; FP32: up to 4, 22^3 248 -> 211, 32^3 287 -> 258, with 7
+  // 40^3 266 -> 328).  Between 17 and 80 blocks the boxes of all blocks are as
+  // fast or faster (11^3 155 us against 212 with clusters of 8).
+  int cluster = 1, fixed_blocks = 0;
+  if (d.S == 1) {
+    const int64_t n = meta_[0].nrow_pad / 32;
+    auto fit = [&](int size, int most, int rows) {
+      for (int r = 1; r <= rows; r++) {
+        const int e = group_resident_entries<T>(opt_.device, r);
+        const int c = std::min(most, group_resident_clusters<T>(r, kCgResidentWarps, e, size));
+        if (e == 0 || c < 1 || (int64_t)c * size * kCgResidentWarps * r < n) continue;
+        cluster = size;
+        fixed_blocks = size * c;
+        R = r;
+        W = std::max(8, (int)((n + (int64_t)fixed_blocks * r - 1) / ((int64_t)fixed_blocks * r)));
+        entries = e;
+        return;
+      }
+    };
+    if (n <= 16 * kCgResidentWarps) fit(16, 1, 1);
+    else if (blocks((int64_t)W * R) > 80) fit(8, 32, sizeof(T) == 4 ? 4 : 2);
+  }
   std::vector<int64_t> aptr(d.nrow / 32 + 1);
   CU(cudaMemcpy(aptr.data(), d.A.ptr, sizeof(int64_t) * aptr.size(), cudaMemcpyDeviceToHost));
   std::vector<int> sim, first(d.S + 1, 0);
@@ -723,7 +749,7 @@ bool TetGroup::resident() {
   for (int s = 0; s < d.S; s++) {
     // cuts of about equal work (entries, and the row's own passes), with at
     // most `per` slices a block
-    const int64_t a = meta_[s].roff / 32, n = meta_[s].nrow_pad / 32, g = (n + per - 1) / per;
+    const int64_t a = meta_[s].roff / 32, n = meta_[s].nrow_pad / 32, g = fixed_blocks ? std::min<int64_t>(n, fixed_blocks) : (n + per - 1) / per;
     auto work = [&](int64_t sl) { return (double)(aptr[sl] - aptr[a]) / 32 + 4.0 * (double)(sl - a); };
     first[s] = (int)sim.size();
     int64_t cut = a;
@@ -738,6 +764,10 @@ bool TetGroup::resident() {
       cut = std::min(next, a + n - (g - 1 - q));
     }
   }
+  while ((int)sim.size() % cluster) {  // blocks without rows fill the last cluster
+    sim.push_back(d.S - 1);
+    s0.push_back(d.nrow / 32);
+  }
   first[d.S] = (int)sim.size();
   s0.push_back(d.nrow / 32);
   // the copy of A: whole slices from the block's first on, as far as they fit
@@ -749,6 +779,7 @@ bool TetGroup::resident() {
     most = std::max(most, cached[b]);
   }
   d.res_blocks = (int)sim.size();
+  d.res_cluster = cluster;
   d.res_warps = W;
   d.res_rows = R;
   d.res_entries = most;

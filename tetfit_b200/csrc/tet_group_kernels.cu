@@ -915,12 +915,12 @@ __global__ void __launch_bounds__(cg_threads<T>(), cg_min_blocks<T>()) grp_cg(Gr
 //   x, r, z       in registers; the pair (z, p_j) is stored for the gathers
 //   exchange      r.r, r.z, which also makes the pairs visible
 //
-// Bound by latency.  24^3 FP64 (97 k rows, 146 blocks of 11 warps): an
-// iteration took 20.6 us with grp_cg and takes 11 us, of which the gathers and
-// products 2.3, the exchanges 3.5 and 4.5 us.  9^3 FP64 (5 k rows, 19 blocks):
-// 14.2 -> 6.1 us.  40^3 FP32 (433 k rows, a third of A streamed): 36 -> 22 us.
-// It beat grp_cg at every size it takes (FP64 to 40^3, 952 -> 805 us a solve;
-// FP32 to 44^3, 955 -> 835 us).
+// Bound by latency.  24^3 FP64 (97 k rows, 120 blocks in clusters of 8): an
+// iteration took 20.6 us with grp_cg and takes 9.5 us, about 2.5 of them the
+// gathers and products, 1 the row updates, the rest the exchanges.  9^3 FP64
+// (5 k rows, one cluster of 16 blocks): 14.2 -> 4.8 us.  40^3 FP32 (433 k rows,
+// 148 blocks, a third of A streamed): 36 -> 22 us.  It beat grp_cg at every
+// size it takes (FP64 to 40^3, 952 -> 805 us a solve; FP32 to 44^3, 955 -> 835).
 template <typename T>
 struct PairOf;
 template <>
@@ -984,7 +984,7 @@ __global__ void __launch_bounds__(32 * kCgResidentWarps, 1) grp_cg_resident(Grou
     cg_bulk_load(sval, (const T*)d.A.val + e0, (uint32_t)cached * (uint32_t)sizeof(T), &sh.bar);
   }
   CgExchange ex{d.res_box, d.res_blocks, d.res_first[s], d.res_first[s + 1] - d.res_first[s], d.err, &sh,
-                (uint32_t)(d.step[s] + 1) * (uint32_t)(2 * d.cg_maxiter + 2)};
+                (uint32_t)(d.step[s] + 1) * (uint32_t)(2 * d.cg_maxiter + 2), d.res_cluster};
   const T* b = (const T*)d.rhs;
   T* x = (T*)d.x;
   const T* pre = (const T*)d.pre;
@@ -1007,14 +1007,17 @@ __global__ void __launch_bounds__(32 * kCgResidentWarps, 1) grp_cg_resident(Grou
     qk[k] = 0;
   }
   __syncthreads();  // the mbarrier is initialised
-  bool alive = cg_bar_wait(&sh.bar);
-  if (!alive) atomicOr(d.err, kBarrierTimedOut);
+  // a copy that does not arrive raises the error flag and a NaN, which ends the
+  // solve in every block at once
+  const bool copied = cg_bar_wait(&sh.bar);
+  if (!copied) atomicOr(d.err, kBarrierTimedOut);
   auto row_dot = [&](int k, auto load, auto form) -> T {
     if (off[k] + 32 * len[k] <= cached)
       return resident_dot<true>(scol + off[k] + lane, sval + off[k] + lane, len[k], load, form);
     return resident_dot<false>(d.A.col + e0 + off[k] + lane, (const T*)d.A.val + e0 + off[k] + lane, len[k], load, form);
   };
-  double v5[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  double v5[5] = {copied ? 0.0 : nan(""), 0.0, 0.0, copied ? 0.0 : nan(""), 0.0};
+  bool alive = true;
   const int64_t i0 = (s0 + warp) * 32 + lane;
 #pragma unroll
   for (int k = 0; k < R; k++) {
@@ -1291,6 +1294,31 @@ int group_resident_entries(int device, int rows) {
   }
   return n;
 }
+// Clusters of `size` blocks that run at once with a resident kernel's full
+// shared memory.
+template <typename T>
+int group_resident_clusters(int rows, int warps, int entries, int size) {
+  auto k = resident_kernel<T>(rows);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(32 * warps);
+  cfg.dynamicSmemBytes = (sizeof(T) + 4) * (size_t)entries;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)size;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+template int group_resident_clusters<float>(int, int, int, int);
+template int group_resident_clusters<double>(int, int, int, int);
 template int group_resident_entries<float>(int, int);
 template int group_resident_entries<double>(int, int);
 
@@ -1362,11 +1390,14 @@ cudaError_t group_launch_step(const GroupDev& d, int cg_blocks, int cg_variant, 
   cfg.blockDim = dim3(resident ? 32 * d.res_warps : cg_threads<T>());
   cfg.dynamicSmemBytes = resident ? (sizeof(T) + 4) * (size_t)d.res_entries : smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)d.res_cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = resident && d.res_cluster > 1 ? 2 : 1;
   cudaError_t err = resident ? cudaLaunchKernelEx(&cfg, resident_kernel<T>(d.res_rows), d)
                     : cg_variant == 0 ? cudaLaunchKernelEx(&cfg, grp_cg<T, true>, d)
                                       : cudaLaunchKernelEx(&cfg, grp_cg<T, false>, d);

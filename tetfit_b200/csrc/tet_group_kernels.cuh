@@ -119,6 +119,7 @@ struct GroupDev {
   // the slices [res_s0[b], res_s0[b + 1]); simulation s has the blocks
   // [res_first[s], res_first[s + 1])
   int res_blocks = 0, res_warps = 0, res_rows = 0, res_entries = 0;  // rows a thread, most copied entries of a block
+  int res_cluster = 1;           // blocks of a cluster
   const int* res_sim = nullptr;
   const int64_t* res_s0 = nullptr;
   const int* res_first = nullptr;
@@ -187,6 +188,8 @@ constexpr int kCgResidentWarps = 16;  // most warps of a block: 128 registers a 
 constexpr int kCgResidentRows = 8;    // most rows of a thread
 template <typename T>
 int group_resident_entries(int device, int rows);
+template <typename T>
+int group_resident_clusters(int rows, int warps, int entries, int size);
 // step_io: this step's carrier values (staging, contiguous) into each
 // running member's carrier row
 cudaError_t group_launch_io_carriers(const GroupDev& d, const double* in, cudaStream_t st);

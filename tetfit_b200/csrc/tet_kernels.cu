@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_resident(DevPtrs d, int ro
   int32_t* scol = reinterpret_cast<int32_t*>(sval + entries);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
   const int n = d.nfree, r0 = blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
-  CgExchange ex{d.box, (int)gridDim.x, 0, (int)gridDim.x, d.err, &sh, 1u};
+  CgExchange ex{d.box, (int)gridDim.x, 0, (int)gridDim.x, d.err, &sh, 1u, 1};
   const double* val = (const double*)d.a_val;
   const double* b = (const double*)d.rhs;
   double* x = (double*)d.x;
