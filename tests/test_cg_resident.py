@@ -33,9 +33,10 @@ def test_resident_equals_general(tmp_path, product_lib, precision, warm):
         c = TetCase(n=n, method=method, split_x=True, eps=(1.0 + 0.2 * i, 2.5), seed=50 + i, steps=40, tolerance=tol)
         return (write_tet_case(os.path.join(str(tmp_path), f"m{i}"), c), 1)
 
-    # 2^3: one slice; 8^3: a few blocks; 17^3 and 21^3: one and two rows a
-    # thread; 36^3: five, part of A streamed in FP64; fem: 19-entry rows
-    groups = [[case(0, 2)], [case(1, 3), case(2, 8), case(3, 5, "fem")], [case(4, 17), case(5, 21)], [case(6, 36)],
+    # 2^3: one slice in a cluster of 16 blocks; 8^3: a few blocks; 17^3 and 21^3:
+    # one and two rows a thread; 36^3: five, part of A streamed in FP64; 24^3 and
+    # 32^3: clusters of 8 (32^3 in FP32 alone); fem: 19-entry rows
+    groups = [[case(0, 2)], [case(9, 9)], [case(10, 24)], [case(11, 32)], [case(1, 3), case(2, 8), case(3, 5, "fem")], [case(4, 17), case(5, 21)], [case(6, 36)],
               [case(7, 15, "fem")]]
     big = case(8, 48)
     opts = dict(precision=precision, warm_start=warm, cg_criterion="rhs", learn_steps=15)

@@ -55,8 +55,11 @@ def check(ptr, col, val, seed, tol=1e-10, guess=False):
     return it, xs
 
 
-@pytest.mark.parametrize("n,long_rows", [(1, 0), (31, 0), (33, 0), (257, 0), (37889, 0), (75777, 0), (151553, 40),
-                                         (40000, 3000), (303105, 0)])
+# flat up to 20480 rows and above 184320, between them clusters of 8 blocks with
+# one row a thread up to 61440 and two up to 122880
+@pytest.mark.parametrize("n,long_rows", [(1, 0), (31, 0), (33, 0), (257, 0), (20480, 0), (20481, 0), (37889, 0),
+                                         (61441, 0), (75777, 0), (122881, 0), (151553, 40), (184321, 0), (40000, 3000),
+                                         (303105, 0)])
 @pytest.mark.parametrize("guess", [False, True])
 def test_solutions(product_lib, n, long_rows, guess):
     check(*spd(n, n, long_rows), seed=n + 1, guess=guess)

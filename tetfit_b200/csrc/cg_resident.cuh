@@ -103,6 +103,15 @@ struct CgExchange {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 
+  // before the first sum(): the block's set-up of shared memory is visible to its
+  // threads, and with clusters every block of the cluster has started
+  __device__ __forceinline__ void enter() {
+    if (cluster > 1)
+      cluster_sync();
+    else
+      __syncthreads();
+  }
+
   // sum() with clusters, from the warps' sums on
   template <int NV, bool kPublish>
   __device__ __forceinline__ void cluster_sum(uint32_t k) {

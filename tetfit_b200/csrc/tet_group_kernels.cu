@@ -1006,7 +1006,7 @@ __global__ void __launch_bounds__(32 * kCgResidentWarps, 1) grp_cg_resident(Grou
     pk[k] = 0;
     qk[k] = 0;
   }
-  __syncthreads();  // the mbarrier is initialised
+  ex.enter();  // the mbarrier is initialised
   // a copy that does not arrive raises the error flag and a NaN, which ends the
   // solve in every block at once
   const bool copied = cg_bar_wait(&sh.bar);

@@ -479,11 +479,12 @@ __global__ void __launch_bounds__(kBlock) tet_cg(DevPtrs d) {
 // pair (z, p) of a column gathered with one load, where p_j = z + beta p_{j-1}
 // is formed with the rounding of the row's owner.  zp (2 n doubles) takes the
 // place of jac and r.  Bound by latency: 131 k rows of 7 entries took 22.8 us an
-// iteration with tet_cg, the call's other costs included, and take 9.5.
+// iteration with tet_cg, the call's other costs included, and take 8.5.
 constexpr int kPcgThreads = 512;
 
 template <int R>
-__global__ void __launch_bounds__(kPcgThreads, 1) pcg_resident(DevPtrs d, int rows_per_block, int entries) {
+__global__ void __launch_bounds__(kPcgThreads, 1) pcg_resident(DevPtrs d, int rows_per_block, int entries,
+                                                              int cluster) {
   constexpr int CH = 7;
   extern __shared__ __align__(16) unsigned char pcg_raw[];
   __shared__ CgShared sh;
@@ -491,8 +492,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_resident(DevPtrs d, int ro
   double* sval = reinterpret_cast<double*>(pcg_raw);
   int32_t* scol = reinterpret_cast<int32_t*>(sval + entries);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
-  const int n = d.nfree, r0 = blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
-  CgExchange ex{d.box, (int)gridDim.x, 0, (int)gridDim.x, d.err, &sh, 1u, 1};
+  const int n = d.nfree, r0 = min(n, (int)blockIdx.x * rows_per_block), r1 = min(n, r0 + rows_per_block);
+  CgExchange ex{d.box, (int)gridDim.x, 0, (int)gridDim.x, d.err, &sh, 1u, cluster};
   const double* val = (const double*)d.a_val;
   const double* b = (const double*)d.rhs;
   double* x = (double*)d.x;
@@ -518,7 +519,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_resident(DevPtrs d, int ro
       if (width[q] >= 0) s += 32 * w;
     }
   }
-  __syncthreads();
+  ex.enter();
   double xk[R], rk[R], pk[R], dk[R], qk[R];
 #pragma unroll
   for (int k = 0; k < R; k++) {
@@ -739,28 +740,67 @@ size_t pcg_box_bytes(int device) {
 bool pcg_resident_fits(int64_t n, int device) { return n <= (int64_t)8 * pcg_sms(device) * kPcgThreads; }
 
 template <int R>
-static cudaError_t pcg_launch_resident(const DevPtrs& d, int device, int sms, cudaStream_t st) {
+static cudaError_t pcg_launch_resident(const DevPtrs& d, int device, int most, int cluster, cudaStream_t st) {
   const int entries = pcg_resident_entries<R>(device);
   if (entries < 1) return cudaErrorLaunchOutOfResources;
-  // as few warps as one block an SM allows, but not fewer than 8
   const int slices = (d.nfree + 31) / 32;
-  int W = (slices + sms * R - 1) / (sms * R);
+  // as few warps as the blocks allow, but not fewer than 8
+  int W = (slices + most * R - 1) / (most * R);
   W = W < 8 ? 8 : W;
-  int rows = 32 * W * R;
-  const int blocks = (d.nfree + rows - 1) / rows;
-  rows = ((slices + blocks - 1) / blocks) * 32;  // evenly
+  // clusters take all their blocks (the last ones may have no rows)
+  int blocks = cluster > 1 ? most : (slices + W * R - 1) / (W * R);
+  const int rows = (slices + blocks - 1) / blocks * 32;  // evenly
+  if (cluster == 1) blocks = (d.nfree + rows - 1) / rows;
   cudaMemsetAsync(d.box, 0, 2 * kCgVals * (size_t)blocks * blocks * sizeof(uint4), st);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((d.nfree + rows - 1) / rows);
+  cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(32 * W);
   cfg.dynamicSmemBytes = (size_t)entries * 12;
   cfg.stream = st;
   cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, pcg_resident<R>, d, rows, entries, cluster);
+}
+
+// Clusters of 8 blocks that run at once with the kernels' full shared memory, no
+// more than one block an SM (the boxes are laid out for that), looked up once for
+// a device.
+constexpr int kPcgClusterRows = 20480;
+static int pcg_clusters(int device) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices];  // one more than the number, 0 not looked up
+  const bool keep = device >= 0 && device < kDevices;
+  if (keep && known[device].load() > 0) return known[device].load() - 1;
+  int n = pcg_sms(device) / 8;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(8);
+  cfg.blockDim = dim3(kPcgThreads);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 8;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, pcg_resident<R>, d, rows, entries);
+  auto look = [&](auto kernel, int entries) {
+    int m = 0;
+    cfg.dynamicSmemBytes = (size_t)entries * 12;
+    if (entries < 1 || cudaOccupancyMaxActiveClusters(&m, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      m = 0;
+    }
+    n = m < n ? m : n;
+  };
+  look(pcg_resident<1>, pcg_resident_entries<1>(device));
+  look(pcg_resident<2>, pcg_resident_entries<2>(device));
+  look(pcg_resident<3>, pcg_resident_entries<3>(device));
+  if (keep) known[device].store(n + 1);
+  return n;
 }
 
 // Standalone FP64 solve.  With boxes (DevPtrs::box) and at most 8 rows a thread
@@ -772,11 +812,23 @@ cudaError_t pcg_launch_solve(DevPtrs d, int blocks, int device, cudaStream_t st)
   cudaMemsetAsync(d.err, 0, sizeof(int), st);
   if (d.box && pcg_resident_fits(d.nfree, device)) {
     const int sms = pcg_sms(device);
+    // Clusters of 8 exchange within themselves through distributed shared memory
+    // first, so 15 blocks instead of 148 poll one another's boxes.  An iteration
+    // on grid matrices takes 6.8 against 7.4 us at 27,000 rows (flat, the same with
+    // 30 blocks: 5.7 against 5.8 us at 15,600 rows, so small systems stay flat), 7.5
+    // against 8.8 at 67,650, 8.5 against 9.4 at 131,150, 8.6 against 14.3 at 162,000.
+    if (d.nfree > kPcgClusterRows) {
+      const int c8 = 8 * pcg_clusters(device);
+      const int64_t per8 = (int64_t)c8 * kPcgThreads;
+      if (d.nfree <= per8) return pcg_launch_resident<1>(d, device, c8, 8, st);
+      if (d.nfree <= 2 * per8) return pcg_launch_resident<2>(d, device, c8, 8, st);
+      if (d.nfree <= 3 * per8) return pcg_launch_resident<3>(d, device, c8, 8, st);
+    }
     const int64_t per = (int64_t)sms * kPcgThreads;  // rows of one row a thread
-    if (d.nfree <= per) return pcg_launch_resident<1>(d, device, sms, st);
-    if (d.nfree <= 2 * per) return pcg_launch_resident<2>(d, device, sms, st);
-    if (d.nfree <= 4 * per) return pcg_launch_resident<4>(d, device, sms, st);
-    return pcg_launch_resident<8>(d, device, sms, st);
+    if (d.nfree <= per) return pcg_launch_resident<1>(d, device, sms, 1, st);
+    if (d.nfree <= 2 * per) return pcg_launch_resident<2>(d, device, sms, 1, st);
+    if (d.nfree <= 4 * per) return pcg_launch_resident<4>(d, device, sms, 1, st);
+    return pcg_launch_resident<8>(d, device, sms, 1, st);
   }
   jacobi_from_csr<<<nblk(d.nfree), kBlock, 0, st>>>(d.a_ptr, d.a_col, (const double*)d.a_val, (double*)d.jac,
                                                     d.nfree);
