@@ -11,6 +11,8 @@
 //   grp_cg         persistent cooperative Jacobi-PCG over every simulation's
 //                  system at once (ConjugateGradientSolver.hpp:52-103), each
 //                  simulation with its own scalars and stopping test
+//   grp_cg_resident  the same for groups that fit one block an SM, rows and
+//                  matrix on chip; grp_finish does the two kernels below after it
 //   grp_scatter    U[free] = x, U[Dirichlet] = source values (:1540-1541)
 //   grp_bump       step counters of the running simulations
 //
