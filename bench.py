@@ -278,9 +278,10 @@ def run_ours(args, rank, world, local_rank):
                      graph_steps=1 if WORKLOADS[args.workload]["kind"] == "fit" and case.n >= 256 else 0)
     setup_s = time.time() - t0
     K, W = args.steps, args.warmup
-    # FIT grids of >= 2 M cells time each kernel variant twice (at most 6
-    # variants) in their first steps before settling: keep those steps in
-    # the warm-up so the timed steps run the chosen kernels
+    # FIT grids of >= 2 M cells whose coefficient classes do not fit time each
+    # kernel variant twice (at most 6 variants) in their first steps before
+    # settling: keep those steps in the warm-up so the timed steps run the
+    # chosen kernels
     tune = 12 if info["method"] == "fdtd" and info["n_cells"] >= 2000000 else 0
     need = W + tune + K + min(K, 50) + 20
     if info["n_steps"] < need:
@@ -389,7 +390,7 @@ def precision_report(script, device, steps=400, every=100):
 # against 709.4 MB algorithmic, fit_h_class 697.6 MB against 708.2 MB.  The ratio is per byte
 # (one plane per block, the same re-use at every size), reported for the
 # dominant kernel as ratio x its algorithmic bytes.
-FIT_DRAM_OVER_ALGORITHMIC = {("fit_e_class", 4): 0.972, ("fit_h_class", 4): 0.985}
+FIT_DRAM_OVER_ALGORITHMIC = {("fit_e_class", 4): 1.009, ("fit_h_class", 4): 0.990}
 FIT_TRAFFIC_NOTE = "ncu DRAM bytes / algorithmic bytes of the kernel at 256^3, times this launch's algorithmic bytes"
 
 

@@ -61,9 +61,11 @@ typedef struct tf_opts {
   int32_t host_threads; /* host threads of the set-up (tf_prepare, tf_batch_open), 0 all */
   int32_t learn_steps;  /* warm_start 3: steps whose solutions train the network
                            (0: 500); the extrapolation is used meanwhile         */
-  int32_t fit_variant;  /* fdtd: 0 automatic (first steps time the variants on grids
-                           of 2 M cells or more), k > 0 forces variant k - 1 for
-                           both halves (all give bitwise identical results)     */
+  int32_t fit_variant;  /* fdtd: 0 automatic (coefficient classes; scenes of more
+                           than 65,535 classes: the first steps time the other
+                           variants on grids of 2 M cells or more), k > 0 forces
+                           variant k - 1 for both halves (all give bitwise
+                           identical results)                                   */
   int32_t file_digits;  /* tf_run: significant digits of the probe files (0: 6, the
                            reference's default stream precision; 17 round-trips) */
   int32_t reserved[2];
@@ -150,7 +152,11 @@ TF_API int tf_step_io(tf_ctx* ctx, const double* carrier_in, double* probe_out, 
 /* Runs up to nsteps steps with CUDA events between kernels and returns the
  * device milliseconds spent per phase: ms[0] sources/BC edges, ms[1] E update,
  * ms[2] source scatter + boundary flux, ms[3] probe export, ms[4] H update
- * (the reference's per-phase averages, Discretization.hpp:2286-2302). */
+ * (the reference's per-phase averages, Discretization.hpp:2286-2302).  Work that
+ * shares a launch counts where the launch is: fdtd with coefficient classes has
+ * the sources in ms[1], flux and probes in ms[4]; dga sources and flux partials
+ * in ms[1], flux sum and probes in ms[3] with the E half; gfdtd and fem as
+ * tf_batch_phase_times. */
 TF_API int tf_phase_times(tf_ctx* ctx, uint64_t nsteps, double* ms5, uint64_t* done);
 /* Whole simulation as RunSimulation does it: prepare, every step, output files. */
 TF_API int tf_run(tf_ctx* ctx, uint32_t sim_label, const tf_opts* opts);
@@ -234,7 +240,7 @@ TF_API int tf_batch_open(const char* const* scripts, const uint32_t* labels, uin
 TF_API int tf_batch_info(tf_batch* b, uint32_t member, tf_info* info);
 /* Advance every unfinished member by up to nsteps steps; *done = the most any member took. */
 TF_API int tf_batch_step(tf_batch* b, uint64_t nsteps, uint64_t* done);
-/* tf_phase_times over the batch: ms5 = H update + probes, sources + rhs, CG, scatter, step end. */
+/* tf_phase_times over the batch: ms5 = H update, sources + probes + rhs, CG, scatter, step end. */
 TF_API int tf_batch_phase_times(tf_batch* b, uint64_t nsteps, double* ms5, uint64_t* done);
 /* One step of every member from host memory: carriers_in holds n_sources values
  * per member in member order (NULL keeps the scripts' waveforms); probes_out
