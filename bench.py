@@ -258,7 +258,8 @@ def roofline_kernel(d, info, es, ms5, nph):
     per_iter = nnz * (4 + es) + n * (13 * es + 8)
     setup = nnz * (4 + es) + n * (8 + 4 * es)
     b = float(its.mean()) * per_iter + setup
-    return "tet_cg", b, ms5[2] / nph, {"cg_iterations_mean": float(its.mean()), "n_free": n, "nnz_A": nnz}
+    name = "grp_cg_resident" if info.get("cg_variant") == 2 else "grp_cg"
+    return name, b, ms5[2] / nph, {"cg_iterations_mean": float(its.mean()), "n_free": n, "nnz_A": nnz}
 
 
 def run_ours(args, rank, world, local_rank):

@@ -3,6 +3,7 @@ memory) against the general CG kernel: members small enough for it alone, then
 again in one batch with a member that makes the group too large for it.  Sizes
 from a few blocks to several rows a thread with part of A streamed."""
 import os
+import threading
 
 import numpy as np
 import pytest
@@ -52,3 +53,33 @@ def test_resident_equals_general(tmp_path, product_lib, precision, warm):
             bound = 1e-10 if precision == "fp64" else 1e-5
             for a, r in zip(gs + (gp, gf), rs + (rp, rf)):
                 assert rel(a, r) <= bound
+
+
+def test_simulations_in_threads(tmp_path, product_lib):
+    """One cluster of 16, clusters of 8 and flat boxes on 148 blocks at once,
+    each from its own thread: the sums have a fixed order, so every state is
+    the one of a run alone, bit for bit."""
+    scripts = [write_tet_case(os.path.join(str(tmp_path), f"t{n}"), TetCase(n=n, method="gfdtd", seed=n, steps=80))
+               for n in (9, 24, 27)]
+
+    def run(script):
+        with tb.Discretization(script) as d:
+            d.prepare(1, precision="fp64")
+            assert d.step(60) == 60
+            return d.state() + (d.solver_stats()[0],)
+
+    alone = [run(s) for s in scripts]
+    got = [None] * len(scripts)
+
+    def work(k):
+        got[k] = run(scripts[k])
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(len(scripts))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for a, g in zip(alone, got):
+        assert g is not None
+        for u, v in zip(a, g):
+            assert np.array_equal(u, v)
