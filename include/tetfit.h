@@ -223,6 +223,19 @@ TF_API int tf_pcg_solve_noalloc(const tf_pcg_args* args, int32_t* iters, double*
  * touched).  Errors through tf_last_error(NULL). */
 TF_API int tf_barrier_check(int32_t device, uint32_t blocks, uint32_t expected, uint32_t rounds,
                             uint32_t timeout_us, int32_t* status, double* ms);
+/* Self-check of the exchange of partial sums in the resident CG kernels; no
+ * reference counterpart.  `blocks` co-resident blocks in clusters of `cluster`
+ * (1: none) form 2 x rounds exchanges numbered from `first` on (the 32-bit
+ * number may wrap) and compare the sums with their exact values.  The last
+ * `absent` blocks (whole clusters) take no part, so that the others' first wait
+ * can never complete.  *status is 0 when every sum is right, 2 when a wait ran
+ * out after timeout_us, 1 when a sum was wrong.  *ms (optional) is the launch's
+ * duration.  Arguments: cluster 1, 2, 4, 8 or 16, blocks a multiple of it, at
+ * most 32 clusters (cluster > 1) and the SM count, first >= 1, 1 <= rounds <=
+ * 100000, absent < blocks, 1 <= timeout_us <= 1000000; otherwise TF_E_ARG
+ * (checked before the GPU is touched).  Errors through tf_last_error(NULL). */
+TF_API int tf_exchange_check(int32_t device, uint32_t blocks, uint32_t cluster, uint32_t first, uint32_t rounds,
+                             uint32_t absent, uint32_t timeout_us, int32_t* status, double* ms);
 /* ---- Batches: many gfdtd simulations advanced together ---------------------
  * The reference runs the simulations of a script one after another
  * (dga_main.cpp:52-62), each with its own mesh, materials, sources and time

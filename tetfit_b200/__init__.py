@@ -99,6 +99,8 @@ _SIGS = {
     "tf_barrier_check": (ctypes.c_int, [ctypes.c_int32, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32,
                                         ctypes.c_uint32, ctypes.POINTER(ctypes.c_int32),
                                         ctypes.POINTER(ctypes.c_double)]),
+    "tf_exchange_check": (ctypes.c_int, [ctypes.c_int32] + [ctypes.c_uint32] * 6 +
+                          [ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_double)]),
     "tf_batch_open": (ctypes.c_int, [ctypes.POINTER(ctypes.c_char_p), ctypes.POINTER(ctypes.c_uint32),
                                      ctypes.c_uint32, ctypes.POINTER(Opts), ctypes.POINTER(_P)]),
     "tf_batch_info": (ctypes.c_int, [_P, ctypes.c_uint32, ctypes.POINTER(Info)]),
@@ -167,6 +169,20 @@ def barrier_check(blocks: int, expected: int, rounds: int = 1, timeout_us: int =
     st = ctypes.c_int32()
     ms = ctypes.c_double()
     rc = lib().tf_barrier_check(device, blocks, expected, rounds, timeout_us, ctypes.byref(st), ctypes.byref(ms))
+    if rc != TF_OK:
+        raise TetfitError(rc, last_thread_error())
+    return st.value, ms.value
+
+
+def exchange_check(blocks: int, cluster: int = 1, first: int = 1, rounds: int = 1, absent: int = 0,
+                   timeout_us: int = 100000, device: int = 0):
+    """Self-check of the resident CG kernels' exchange of partial sums
+    (tf_exchange_check): (status, ms) of one launch.  status 0: every sum was
+    right; 2: a wait ran out of time (absent blocks); 1: a sum was wrong."""
+    st = ctypes.c_int32()
+    ms = ctypes.c_double()
+    rc = lib().tf_exchange_check(device, blocks, cluster, first, rounds, absent, timeout_us, ctypes.byref(st),
+                                 ctypes.byref(ms))
     if rc != TF_OK:
         raise TetfitError(rc, last_thread_error())
     return st.value, ms.value

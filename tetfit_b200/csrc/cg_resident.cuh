@@ -12,6 +12,12 @@
 // in exchange k + 2, after it has read every record of k + 1, whose writers had
 // read theirs of k.  Every block of a system is resident (cooperative launch),
 // and a wait is bounded like the grid barrier's (grid_barrier.cuh).
+//
+// Exchanges are numbered from 1 (cleared boxes hold 0) and go on from solve to
+// solve when the boxes are not cleared in between; the number may wrap.  A solve
+// of `it` iterations takes 2 it + 1 exchanges, an odd count, so the sets take
+// turns at a solve's first exchange and every record in use is written again
+// within two solves: a wrapped number meets no record of its last time round.
 #pragma once
 #include <cstdint>
 
@@ -56,6 +62,7 @@ struct CgExchange {
   CgShared* sh;
   uint32_t round;   // number of the next exchange
   int cluster;      // blocks of a cluster, 1 none
+  uint64_t limit_ns = kBarrierLimitNs;
 
   // Waits for the record of exchange k at p; false when it ran out.
   template <bool kAcquire>
@@ -80,7 +87,7 @@ struct CgExchange {
       if ((n & 255) == 255) {  // no clock read in a wait that ends at once
         const uint64_t now = global_ns();
         if (t0 == 0) t0 = now;
-        if (*(volatile int*)err != 0 || now - t0 > kBarrierLimitNs) {
+        if (*(volatile int*)err != 0 || now - t0 > limit_ns) {
           atomicOr(err, kBarrierTimedOut);
           return false;
         }

@@ -787,22 +787,33 @@ bool TetGroup::resident() {
   d.res_sim = (const int*)upload(sim);
   d.res_s0 = (const int64_t*)upload(s0);
   d.res_first = (const int*)upload(first);
-  const size_t boxes = (size_t)2 * 5 * sim.size() * sim.size() * 16;
-  d.res_box = (uint4*)dalloc(boxes);
-  CU(cudaMemset(d.res_box, 0, boxes));
+  d.res_box = (uint4*)dalloc(exchange_bytes());
+  d.res_round = (uint32_t*)dalloc(sizeof(uint32_t) * (size_t)d.S);
+  reset_exchange();
   d.zp = dalloc((size_t)(opt_.warm_start == 3 ? 4 : 2) * (size_t)d.nrow * sizeof(T));
   cg_blocks_ = d.res_blocks;
   return true;
 }
 
-// A grid-barrier timeout in the CG kernel leaves the step's results invalid:
-// report it (and reset the barrier so the group can be closed cleanly).
+size_t TetGroup::exchange_bytes() const { return (size_t)2 * 5 * dev_.res_blocks * dev_.res_blocks * sizeof(uint4); }
+
+// Cleared boxes and exchange numbers from 1.
+void TetGroup::reset_exchange() {
+  const std::vector<uint32_t> one(dev_.S, 1u);
+  CU(cudaMemset(dev_.res_box, 0, exchange_bytes()));
+  CU(cudaMemcpy(dev_.res_round, one.data(), sizeof(uint32_t) * one.size(), cudaMemcpyHostToDevice));
+}
+
+// A wait that ran out in the CG kernel leaves the step's results invalid:
+// report it (and reset the barrier or the boxes, whose blocks may have stopped
+// at different exchanges, so the group can be closed cleanly).
 void TetGroup::check_err() {
   int e = 0;
   CU(cudaMemcpy(&e, dev_.err, sizeof(int), cudaMemcpyDeviceToHost));
   if (!e) return;
   CU(cudaMemset(dev_.err, 0, sizeof(int)));
   CU(cudaMemset(dev_.gbar, 0, 2 * sizeof(unsigned int)));
+  if (dev_.res_box) reset_exchange();
   throw CudaError("CG kernel: a grid barrier wait ran out of time; the step's results are not valid");
 }
 

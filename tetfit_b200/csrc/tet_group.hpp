@@ -79,6 +79,8 @@ class TetGroup {
   void partition();
   template <typename T>
   bool resident();
+  size_t exchange_bytes() const;
+  void reset_exchange();
   void check_err();
   void launch(int n, cudaEvent_t* ev);
   void capture_graph(int len);

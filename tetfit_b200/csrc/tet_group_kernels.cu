@@ -986,7 +986,7 @@ __global__ void __launch_bounds__(32 * kCgResidentWarps, 1) grp_cg_resident(Grou
     cg_bulk_load(sval, (const T*)d.A.val + e0, (uint32_t)cached * (uint32_t)sizeof(T), &sh.bar);
   }
   CgExchange ex{d.res_box, d.res_blocks, d.res_first[s], d.res_first[s + 1] - d.res_first[s], d.err, &sh,
-                (uint32_t)(d.step[s] + 1) * (uint32_t)(2 * d.cg_maxiter + 2), d.res_cluster};
+                d.res_round[s], d.res_cluster};
   const T* b = (const T*)d.rhs;
   T* x = (T*)d.x;
   const T* pre = (const T*)d.pre;
@@ -1119,8 +1119,8 @@ __global__ void __launch_bounds__(32 * kCgResidentWarps, 1) grp_cg_resident(Grou
   }
 }
 
-// The Dirichlet edges' source values and the step counters (after
-// grp_cg_resident, which scatters the solution itself).
+// The Dirichlet edges' source values, the exchange numbers and the step counters
+// (after grp_cg_resident, which scatters the solution itself).
 template <typename T>
 __global__ void __launch_bounds__(kGB) grp_finish(GroupDev d) {
   const int64_t k = (int64_t)blockIdx.x * kGB + threadIdx.x;
@@ -1129,7 +1129,10 @@ __global__ void __launch_bounds__(kGB) grp_finish(GroupDev d) {
     if (d.Uo) ((T*)d.Uo)[e] = ((const T*)d.U)[e];
     ((T*)d.U)[e] = ((const T*)d.src)[e];
   }
-  if (k < d.S && d.step[k] < d.nsteps[k]) d.step[k] += 1;
+  if (k < d.S && d.step[k] < d.nsteps[k]) {
+    d.res_round[k] += 2u * (uint32_t)d.cg_iters[d.stat_off[k] + d.step[k]] + 1u;
+    d.step[k] += 1;
+  }
 }
 
 // Leapfrog energy of member s in the state after a step, (U^n, B^{n-1/2}):

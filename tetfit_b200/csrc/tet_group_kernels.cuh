@@ -125,6 +125,7 @@ struct GroupDev {
   const int* res_first = nullptr;
   const int* res_cached = nullptr;  // entries of A a block copies (whole slices)
   uint4* res_box = nullptr;      // exchange boxes (cg_resident.cuh)
+  uint32_t* res_round = nullptr; // per simulation: number of its next exchange
   void* zp = nullptr;            // pairs (z, p) of the rows, once more for the second start of warm_start 3
   int cg_maxiter = 100, cg_criterion = 0, warm_start = 0;
   // learned warm start (warm_start 3): the network's guess goes to x, the
