@@ -1116,11 +1116,12 @@ __global__ void __launch_bounds__(32 * kCgResidentWarps, 1) grp_cg_resident(Grou
     d.cg_resid[k] = res / res0;
     d.cg_limit[k] = unmet() ? 1 : 0;
     if (d.kept) d.kept[k] = dual && !sel ? 1 : 0;
+    d.res_round[s] = ex.round;  // every block read it before its first record
   }
 }
 
-// The Dirichlet edges' source values, the exchange numbers and the step counters
-// (after grp_cg_resident, which scatters the solution itself).
+// The Dirichlet edges' source values and the step counters (after
+// grp_cg_resident, which scatters the solution itself).
 template <typename T>
 __global__ void __launch_bounds__(kGB) grp_finish(GroupDev d) {
   const int64_t k = (int64_t)blockIdx.x * kGB + threadIdx.x;
@@ -1129,10 +1130,7 @@ __global__ void __launch_bounds__(kGB) grp_finish(GroupDev d) {
     if (d.Uo) ((T*)d.Uo)[e] = ((const T*)d.U)[e];
     ((T*)d.U)[e] = ((const T*)d.src)[e];
   }
-  if (k < d.S && d.step[k] < d.nsteps[k]) {
-    d.res_round[k] += 2u * (uint32_t)d.cg_iters[d.stat_off[k] + d.step[k]] + 1u;
-    d.step[k] += 1;
-  }
+  if (k < d.S && d.step[k] < d.nsteps[k]) d.step[k] += 1;
 }
 
 // Leapfrog energy of member s in the state after a step, (U^n, B^{n-1/2}):
