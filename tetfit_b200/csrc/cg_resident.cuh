@@ -4,10 +4,12 @@
 // latency: the two inner products of an iteration each end in an exchange of
 // partial sums between every block of the system.  Here a block publishes its
 // partial as one 16-byte record, a double in two 8-byte words of 32 data bits
-// and the 32-bit number of the exchange, so that a record announces itself (an
-// 8-byte word is written at once), and every block polls the records of its
-// system and adds them in a fixed order: one store and one load through L2
-// instead of an atomic counter, a generation word and a read of the partials.
+// and the 32-bit number of the exchange, so that a record announces itself (the
+// line format of NCCL's low-latency protocol; the vector accesses below are of
+// 8-byte elements, each of which the memory model writes and reads whole), and
+// every block polls the records of its system and adds them in a fixed order:
+// one store and one load through L2 instead of an atomic counter, a generation
+// word and a read of the partials.
 // Records alternate between two sets: a block overwrites the set of exchange k
 // in exchange k + 2, after it has read every record of k + 1, whose writers had
 // read theirs of k.  Every block of a system is resident (cooperative launch),
@@ -69,19 +71,13 @@ struct CgExchange {
   __device__ __forceinline__ bool read(const uint4* p, uint32_t k, double& a) {
     uint64_t t0 = 0;
     for (uint32_t n = 0;; n++) {
-      uint32_t x, fx, y, fy;
+      uint64_t lo, hi;  // data in the lower half, number in the upper
       if (kAcquire)
-        asm volatile("ld.acquire.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(x), "=r"(fx), "=r"(y), "=r"(fy)
-                     : "l"(p)
-                     : "memory");
+        asm volatile("ld.acquire.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
       else
-        asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(x), "=r"(fx), "=r"(y), "=r"(fy)
-                     : "l"(p)
-                     : "memory");
-      if (fx == k && fy == k) {
-        a = __hiloint2double((int)y, (int)x);
+        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+      if ((uint32_t)(lo >> 32) == k && (uint32_t)(hi >> 32) == k) {
+        a = __hiloint2double((int)(uint32_t)hi, (int)(uint32_t)lo);
         return true;
       }
       if ((n & 255) == 255) {  // no clock read in a wait that ends at once
@@ -95,8 +91,9 @@ struct CgExchange {
     }
   }
   __device__ __forceinline__ void write(uint4* p, uint32_t k, double a) {
-    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"((uint32_t)__double2loint(a)),
-                 "r"(k), "r"((uint32_t)__double2hiint(a)), "r"(k)
+    const uint64_t tag = (uint64_t)k << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(tag | (uint32_t)__double2loint(a)),
+                 "l"(tag | (uint32_t)__double2hiint(a))
                  : "memory");
   }
   static __device__ __forceinline__ uint32_t peer(const void* p, int rank) {
@@ -156,6 +153,14 @@ struct CgExchange {
   // v[] becomes the sums over the system's threads.  With kPublish, global
   // stores made before the call by any thread of the system are visible to
   // every thread after it.  False when a wait ran out.
+  //
+  // Without it (the p.q sum) the records still keep the threads' gathers of the
+  // pairs before the owners' next stores of them: every gathered value is a term
+  // of the sum, so its load has returned before the thread's part of the record
+  // is written, and an owner stores after its loop on the records has ended.
+  // That is a chain of data and control dependencies, not a release and an
+  // acquire, which the memory model asks for and which cost 336 us a step
+  // against 319 at 28^3 FP64 (24^3 264 / 261, 40^3 FP32 564 / 556).
   template <int NV, bool kPublish>
   __device__ __forceinline__ bool sum(double (&v)[NV]) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
