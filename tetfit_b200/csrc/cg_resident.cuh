@@ -24,13 +24,9 @@
 #include <cstdint>
 
 #include "grid_barrier.cuh"
+#include "resident_choice.hpp"
 
 namespace tf {
-
-constexpr int kCgVals = 5;     // most values of an exchange
-constexpr int kCgChunks = 10;  // 32-block chunks of a system
-
-constexpr int kCgCluster = 16;  // most blocks of a cluster
 
 struct CgShared {
   double warp[kCgVals][32];

@@ -17,7 +17,6 @@ namespace tf {
 
 namespace {
 
-constexpr int kCgMaxChunksHost = 10;  // kCgMaxChunks of cg_resident.cuh
 constexpr int kTuneSteps = 10;  // 2 warm-up steps, then 4 timed steps per CG variant
 int64_t up32(int64_t n) { return (n + 31) & ~int64_t(31); }
 
@@ -695,52 +694,34 @@ void TetGroup::partition() {
 // 955), and gives the same iterates but for the order of the sums.
 template <typename T>
 bool TetGroup::resident() {
-  GroupDev& d = dev_;
   int sms = 0;
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt_.device));
-  sms = std::min(sms, 32 * kCgMaxChunksHost);
-  auto blocks = [&](int64_t per) {
-    int64_t g = 0;
-    for (const Meta& m : meta_) g += (m.nrow_pad / 32 + per - 1) / per;
-    return g;
-  };
-  for (const Meta& m : meta_)
-    if (m.nrow_pad == 0) return false;
-  // rows a thread: as few as keep one block an SM, and then as few warps, but
-  // not fewer than 8: the exchanges of a small system stay between a few blocks
-  int R = 1;
-  while (R <= kCgResidentRows && blocks((int64_t)kCgResidentWarps * R) > sms) R++;
-  if (R > kCgResidentRows) return false;
-  int W = 8;
-  while (W < kCgResidentWarps && blocks((int64_t)W * R) > sms) W++;
-  int entries = group_resident_entries<T>(opt_.device, R);
-  if (entries == 0) return false;
-  // Clusters (one simulation): one of 16 blocks when the rows fit it, a row a
-  // thread (9^3 FP64 141 -> 120 us a solve); as many of 8 as run at once, 15 on
-  // 148 SMs, when the exchange is between more than 80 blocks and the rows a
-  // thread are few (FP64: up to 2, 16^3 212 -> 184 us, 24^3 285 -> 244, with 3
-  // 27^3 293 -> 311; FP32: up to 4, 22^3 248 -> 211, 32^3 287 -> 258, with 7
-  // 40^3 266 -> 328).  Between 17 and 80 blocks the boxes of all blocks are as
-  // fast or faster (11^3 155 us against 212 with clusters of 8).
-  int cluster = 1, fixed_blocks = 0;
-  if (d.S == 1) {
-    const int64_t n = meta_[0].nrow_pad / 32;
-    auto fit = [&](int size, int most, int rows) {
-      for (int r = 1; r <= rows; r++) {
-        const int e = group_resident_entries<T>(opt_.device, r);
-        const int c = std::min(most, group_resident_clusters<T>(r, kCgResidentWarps, e, size));
-        if (e == 0 || c < 1 || (int64_t)c * size * kCgResidentWarps * r < n) continue;
-        cluster = size;
-        fixed_blocks = size * c;
-        R = r;
-        W = std::max(8, (int)((n + (int64_t)fixed_blocks * r - 1) / ((int64_t)fixed_blocks * r)));
-        entries = e;
-        return;
-      }
-    };
-    if (n <= 16 * kCgResidentWarps) fit(16, 1, 1);
-    else if (blocks((int64_t)W * R) > 80) fit(8, 32, sizeof(T) == 4 ? 4 : 2);
+  std::vector<int64_t> slices;
+  for (const Meta& m : meta_) slices.push_back(m.nrow_pad / 32);
+  const auto choices = group_choices(
+      slices, sms, sizeof(T) == 4, [&](int rows) { return group_resident_entries<T>(opt_.device, rows); },
+      [&](int rows, int entries, int size) {
+        return group_resident_clusters<T>(rows, kCgResidentWarps, entries, size);
+      });
+  // each is launched once with nothing to do: one the device refuses, though its
+  // queries allow it, leaves the next
+  for (const ResidentChoice& c : choices) {
+    lay_out_resident<T>(c);
+    if (group_resident_trial<T>(dev_, stream_) == cudaSuccess) {
+      cg_blocks_ = dev_.res_blocks;
+      return true;
+    }
+    cudaGetLastError();
   }
+  dev_.res_box = nullptr;
+  return false;
+}
+
+template <typename T>
+void TetGroup::lay_out_resident(const ResidentChoice& choice) {
+  GroupDev& d = dev_;
+  const int W = choice.warps, R = choice.rows, cluster = choice.cluster, fixed_blocks = choice.blocks,
+            entries = choice.entries;
   std::vector<int64_t> aptr(d.nrow / 32 + 1);
   CU(cudaMemcpy(aptr.data(), d.A.ptr, sizeof(int64_t) * aptr.size(), cudaMemcpyDeviceToHost));
   std::vector<int> sim, first(d.S + 1, 0);
@@ -791,11 +772,9 @@ bool TetGroup::resident() {
   d.res_round = (uint32_t*)dalloc(sizeof(uint32_t) * (size_t)d.S);
   reset_exchange();
   d.zp = dalloc((size_t)(opt_.warm_start == 3 ? 4 : 2) * (size_t)d.nrow * sizeof(T));
-  cg_blocks_ = d.res_blocks;
-  return true;
 }
 
-size_t TetGroup::exchange_bytes() const { return (size_t)2 * 5 * dev_.res_blocks * dev_.res_blocks * sizeof(uint4); }
+size_t TetGroup::exchange_bytes() const { return cg_box_bytes((size_t)dev_.res_blocks); }
 
 // Cleared boxes and exchange numbers from 1.
 void TetGroup::reset_exchange() {

@@ -79,6 +79,8 @@ class TetGroup {
   void partition();
   template <typename T>
   bool resident();
+  template <typename T>
+  void lay_out_resident(const ResidentChoice& choice);
   size_t exchange_bytes() const;
   void reset_exchange();
   void check_err();

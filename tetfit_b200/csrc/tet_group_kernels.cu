@@ -1320,6 +1320,30 @@ int group_resident_clusters(int rows, int warps, int entries, int size) {
   }
   return n;
 }
+template <typename T>
+static cudaError_t launch_resident(const GroupDev& d, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(d.res_blocks);
+  cfg.blockDim = dim3(32 * d.res_warps);
+  cfg.dynamicSmemBytes = (sizeof(T) + 4) * (size_t)d.res_entries;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)d.res_cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = d.res_cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, resident_kernel<T>(d.res_rows), d);
+}
+template <typename T>
+cudaError_t group_resident_trial(GroupDev d, cudaStream_t st) {
+  d.nsteps = d.step;  // no simulation has a step to make: every block returns
+  return launch_resident<T>(d, st);
+}
+template cudaError_t group_resident_trial<float>(GroupDev, cudaStream_t);
+template cudaError_t group_resident_trial<double>(GroupDev, cudaStream_t);
 template int group_resident_clusters<float>(int, int, int, int);
 template int group_resident_clusters<double>(int, int, int, int);
 template int group_resident_entries<float>(int, int);
@@ -1387,23 +1411,23 @@ cudaError_t group_launch_step(const GroupDev& d, int cg_blocks, int cg_variant, 
     }
   }
   if (ev) cudaEventRecord(ev[2], st);
-  cudaLaunchConfig_t cfg = {};
   const bool resident = cg_variant == kCgResident;
-  cfg.gridDim = dim3(resident ? d.res_blocks : cg_blocks);
-  cfg.blockDim = dim3(resident ? 32 * d.res_warps : cg_threads<T>());
-  cfg.dynamicSmemBytes = resident ? (sizeof(T) + 4) * (size_t)d.res_entries : smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)d.res_cluster;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = resident && d.res_cluster > 1 ? 2 : 1;
-  cudaError_t err = resident ? cudaLaunchKernelEx(&cfg, resident_kernel<T>(d.res_rows), d)
-                    : cg_variant == 0 ? cudaLaunchKernelEx(&cfg, grp_cg<T, true>, d)
-                                      : cudaLaunchKernelEx(&cfg, grp_cg<T, false>, d);
+  cudaError_t err;
+  if (resident) {
+    err = launch_resident<T>(d, st);
+  } else {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cg_blocks);
+    cfg.blockDim = dim3(cg_threads<T>());
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    err = cg_variant == 0 ? cudaLaunchKernelEx(&cfg, grp_cg<T, true>, d) : cudaLaunchKernelEx(&cfg, grp_cg<T, false>, d);
+  }
   if (err != cudaSuccess) return err;
   if (ev) cudaEventRecord(ev[3], st);
   if (resident) {

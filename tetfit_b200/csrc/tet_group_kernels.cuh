@@ -27,6 +27,8 @@
 
 #include <cstdint>
 
+#include "resident_choice.hpp"
+
 namespace tf {
 
 constexpr int32_t kPadCol = 0x7fffffff;
@@ -185,12 +187,13 @@ cudaError_t group_launch_step(const GroupDev& d, int cg_blocks, int cg_variant, 
 template <typename T>
 int group_cg_blocks(int device, int S, size_t* smem);
 constexpr int kCgResident = 2;      // CG variant: 0 fused, 1 three barriers, 2 resident
-constexpr int kCgResidentWarps = 16;  // most warps of a block: 128 registers a thread hold up to 8 rows
-constexpr int kCgResidentRows = 8;    // most rows of a thread
 template <typename T>
 int group_resident_entries(int device, int rows);
 template <typename T>
 int group_resident_clusters(int rows, int warps, int entries, int size);
+// a launch of grp_cg_resident as a step makes it, with every simulation at rest
+template <typename T>
+cudaError_t group_resident_trial(GroupDev d, cudaStream_t st);
 // step_io: this step's carrier values (staging, contiguous) into each
 // running member's carrier row
 cudaError_t group_launch_io_carriers(const GroupDev& d, const double* in, cudaStream_t st);

@@ -480,8 +480,6 @@ __global__ void __launch_bounds__(kBlock) tet_cg(DevPtrs d) {
 // is formed with the rounding of the row's owner.  zp (2 n doubles) takes the
 // place of jac and r.  Bound by latency: 131 k rows of 7 entries took 22.8 us an
 // iteration with tet_cg, the call's other costs included, and take 8.5.
-constexpr int kPcgThreads = 512;
-
 template <int R>
 __global__ void __launch_bounds__(kPcgThreads, 1) pcg_resident(DevPtrs d, int rows_per_block, int entries,
                                                               int cluster) {
@@ -715,13 +713,17 @@ static int pcg_resident_entries(int device) {
   int most = 0, per_sm = 0;
   cudaFuncAttributes fa{};
   if (cudaFuncGetAttributes(&fa, pcg_resident<R>) != cudaSuccess ||
-      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
+    cudaGetLastError();
     return 0;
+  }
   const int entries = (most - (int)fa.sharedSizeBytes) / (12 * 32) * 32;
   if (cudaFuncSetAttribute(pcg_resident<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, entries * 12) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_resident<R>, kPcgThreads, entries * 12) != cudaSuccess ||
-      per_sm < 1)
+      per_sm < 1) {
+    cudaGetLastError();
     return 0;
+  }
   if (keep) known[device].store(entries);
   return entries;
 }
@@ -731,47 +733,55 @@ static int pcg_sms(int device) {
   return sms < 32 * kCgChunks ? sms : 32 * kCgChunks;
 }
 // bytes of DevPtrs::box
-size_t pcg_box_bytes(int device) {
-  const size_t g = (size_t)pcg_sms(device);
-  return 2 * kCgVals * g * g * sizeof(uint4);
+size_t pcg_box_bytes(int device) { return cg_box_bytes((size_t)pcg_sms(device)); }
+
+static int pcg_entries(int rows, int device) {
+  switch (rows) {
+    case 1: return pcg_resident_entries<1>(device);
+    case 2: return pcg_resident_entries<2>(device);
+    case 3: return pcg_resident_entries<3>(device);
+    case 4: return pcg_resident_entries<4>(device);
+    default: return pcg_resident_entries<8>(device);
+  }
+}
+static ResidentChoice pcg_flat_choice(int64_t n, int device) {
+  return pcg_flat(n, pcg_sms(device), [&](int rows) { return pcg_entries(rows, device); });
 }
 
 // whether pcg_launch_solve takes the resident kernel (given boxes)
-bool pcg_resident_fits(int64_t n, int device) { return n <= (int64_t)8 * pcg_sms(device) * kPcgThreads; }
+bool pcg_resident_fits(int64_t n, int device) { return pcg_flat_choice(n, device).rows > 0; }
 
-template <int R>
-static cudaError_t pcg_launch_resident(const DevPtrs& d, int device, int most, int cluster, cudaStream_t st) {
-  const int entries = pcg_resident_entries<R>(device);
-  if (entries < 1) return cudaErrorLaunchOutOfResources;
+static cudaError_t pcg_launch_resident(const DevPtrs& d, const ResidentChoice& c, cudaStream_t st) {
   const int slices = (d.nfree + 31) / 32;
-  // as few warps as the blocks allow, but not fewer than 8
-  int W = (slices + most * R - 1) / (most * R);
-  W = W < 8 ? 8 : W;
-  // clusters take all their blocks (the last ones may have no rows)
-  int blocks = cluster > 1 ? most : (slices + W * R - 1) / (W * R);
-  const int rows = (slices + blocks - 1) / blocks * 32;  // evenly
-  if (cluster == 1) blocks = (d.nfree + rows - 1) / rows;
-  cudaMemsetAsync(d.box, 0, 2 * kCgVals * (size_t)blocks * blocks * sizeof(uint4), st);
+  const int rows = (slices + c.blocks - 1) / c.blocks * 32;  // evenly
+  const int blocks = c.cluster > 1 ? c.blocks : (d.nfree + rows - 1) / rows;
+  cudaMemsetAsync(d.box, 0, cg_box_bytes((size_t)blocks), st);
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.x = (unsigned)c.cluster;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(32 * W);
-  cfg.dynamicSmemBytes = (size_t)entries * 12;
+  cfg.blockDim = dim3(32 * c.warps);
+  cfg.dynamicSmemBytes = (size_t)c.entries * 12;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, pcg_resident<R>, d, rows, entries, cluster);
+  cfg.numAttrs = c.cluster > 1 ? 2 : 1;
+  auto launch = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, d, rows, c.entries, c.cluster); };
+  switch (c.rows) {
+    case 1: return launch(pcg_resident<1>);
+    case 2: return launch(pcg_resident<2>);
+    case 3: return launch(pcg_resident<3>);
+    case 4: return launch(pcg_resident<4>);
+    default: return launch(pcg_resident<8>);
+  }
 }
 
 // Clusters of 8 blocks that run at once with the kernels' full shared memory, no
 // more than one block an SM (the boxes are laid out for that), looked up once for
 // a device.
-constexpr int kPcgClusterRows = 20480;
 static int pcg_clusters(int device) {
   constexpr int kDevices = 64;
   static std::atomic<int> known[kDevices];  // one more than the number, 0 not looked up
@@ -805,30 +815,18 @@ static int pcg_clusters(int device) {
 
 // Standalone FP64 solve.  With boxes (DevPtrs::box) and at most 8 rows a thread
 // the resident kernel, which beat tet_cg at every size it takes (rows of 7
-// entries, us an iteration of a call: 1 k rows 5.3 against 21.1, 131 k 9.5
-// against 22.8, 594 k 31.8 against 35.8); otherwise preconditioner, then the
-// persistent PCG kernel.
+// entries, us an iteration of a call: 1 k rows 5.3 against 21.1, 131 k 8.5
+// against 22.8, 594 k 31.8 against 35.8); otherwise, and where the device does
+// not give it its shared memory, preconditioner, then the persistent PCG kernel.
 cudaError_t pcg_launch_solve(DevPtrs d, int blocks, int device, cudaStream_t st) {
   cudaMemsetAsync(d.err, 0, sizeof(int), st);
-  if (d.box && pcg_resident_fits(d.nfree, device)) {
-    const int sms = pcg_sms(device);
-    // Clusters of 8 exchange within themselves through distributed shared memory
-    // first, so 15 blocks instead of 148 poll one another's boxes.  An iteration
-    // on grid matrices takes 6.8 against 7.4 us at 27,000 rows (flat, the same with
-    // 30 blocks: 5.7 against 5.8 us at 15,600 rows, so small systems stay flat), 7.5
-    // against 8.8 at 67,650, 8.5 against 9.4 at 131,150, 8.6 against 14.3 at 162,000.
-    if (d.nfree > kPcgClusterRows) {
-      const int c8 = 8 * pcg_clusters(device);
-      const int64_t per8 = (int64_t)c8 * kPcgThreads;
-      if (d.nfree <= per8) return pcg_launch_resident<1>(d, device, c8, 8, st);
-      if (d.nfree <= 2 * per8) return pcg_launch_resident<2>(d, device, c8, 8, st);
-      if (d.nfree <= 3 * per8) return pcg_launch_resident<3>(d, device, c8, 8, st);
-    }
-    const int64_t per = (int64_t)sms * kPcgThreads;  // rows of one row a thread
-    if (d.nfree <= per) return pcg_launch_resident<1>(d, device, sms, 1, st);
-    if (d.nfree <= 2 * per) return pcg_launch_resident<2>(d, device, sms, 1, st);
-    if (d.nfree <= 4 * per) return pcg_launch_resident<4>(d, device, sms, 1, st);
-    return pcg_launch_resident<8>(d, device, sms, 1, st);
+  const ResidentChoice flat = d.box ? pcg_flat_choice(d.nfree, device) : ResidentChoice();
+  if (flat.rows) {
+    const ResidentChoice c = pcg_clustered(
+        d.nfree, [&] { return pcg_clusters(device); }, [&](int rows) { return pcg_entries(rows, device); });
+    if (c.rows && pcg_launch_resident(d, c, st) == cudaSuccess) return cudaSuccess;
+    if (c.rows) cudaGetLastError();  // a cluster launch the device refused
+    return pcg_launch_resident(d, flat, st);
   }
   jacobi_from_csr<<<nblk(d.nfree), kBlock, 0, st>>>(d.a_ptr, d.a_col, (const double*)d.a_val, (double*)d.jac,
                                                     d.nfree);
