@@ -1,9 +1,11 @@
-// Error types and the CUDA-call check used across the host runtime.
+// Error types, the CUDA-call check and the graph calls used across the host runtime.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <stdexcept>
 #include <string>
+
+#include "step_graph.hpp"
 
 namespace tf {
 
@@ -22,6 +24,18 @@ inline void cuda_check(cudaError_t e, const char* what, const char* file, int li
     throw CudaError(std::string(what) + " failed at " + file + ":" + std::to_string(line) + ": " +
                     cudaGetErrorString(e));
 }
+
+// Graph calls of capture_steps.
+struct CudaGraphs {
+  using Stream = cudaStream_t;
+  using Graph = cudaGraph_t;
+  using Exec = cudaGraphExec_t;
+  static bool begin(Stream s) { return cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess; }
+  static bool end(Stream s, Graph* g) { return cudaStreamEndCapture(s, g) == cudaSuccess; }
+  static bool instantiate(Exec* x, Graph g) { return cudaGraphInstantiate(x, g, 0) == cudaSuccess; }
+  static void destroy(Graph g) { cudaGraphDestroy(g); }
+  static void clear_error() { cudaGetLastError(); }
+};
 
 }  // namespace tf
 

@@ -173,6 +173,7 @@ class FitSim : public Sim {
   // graphs
   cudaGraphExec_t graph_ = nullptr;
   int graph_len_ = 0;
+  bool graph_failed_ = false;  // a capture was refused: steps are launched one by one
   // reference numbering maps (built on demand): comp << 60 | slot
   std::vector<int64_t> edge_map_, face_map_;
 };

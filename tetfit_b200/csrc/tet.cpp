@@ -2030,13 +2030,9 @@ uint64_t TetSim::step(uint64_t n) {
   // every step launches the same kernels with the same arguments: runs of glen
   // steps replay one captured graph, captured before the timed region opens
   const int glen = opt_.graph_steps > 0 ? opt_.graph_steps : 16;
-  if (glen > 1 && n >= (uint64_t)glen && !graph_) {
-    cudaGraph_t g;
-    CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    launch_steps(glen, nullptr);
-    CU(cudaStreamEndCapture(stream_, &g));
-    CU(cudaGraphInstantiate(&graph_, g, 0));
-    CU(cudaGraphDestroy(g));
+  if (glen > 1 && n >= (uint64_t)glen && !graph_ && !graph_failed_) {
+    graph_ = capture_steps<CudaGraphs>(stream_, [&] { launch_steps(glen, nullptr); });
+    graph_failed_ = !graph_;
   }
   CU(cudaEventRecord(ev0_, stream_));
   uint64_t left = n;

@@ -181,6 +181,7 @@ class TetSim : public Sim {
   const int32_t *dedge_new_ = nullptr, *dface_new_ = nullptr;
   double* dexport_ = nullptr;                      // a field on its way to the host
   cudaGraphExec_t graph_ = nullptr;
+  bool graph_failed_ = false;                      // a capture was refused: steps are launched one by one
   double* pinned_ = nullptr;
   // gfdtd runs on the group engine (a group of one simulation)
   std::unique_ptr<TetGroup> group_;

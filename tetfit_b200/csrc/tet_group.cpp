@@ -897,30 +897,10 @@ uint64_t TetGroup::step(uint64_t n) {
 // the runtime refuses leaves graph_exec_ null and graph_failed_ set; the
 // steps are then launched one by one (same kernels, same results).
 void TetGroup::capture_graph(int len) {
-  cudaGraph_t g = nullptr;
-  if (cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-    cudaGetLastError();
-    graph_failed_ = true;
-    return;
-  }
   const int64_t before = launched_;
-  bool ok = true;
-  try {
-    launch(len, nullptr);
-  } catch (const CudaError&) {
-    ok = false;  // a launch the capture refused; end the capture below
-  }
+  graph_exec_ = capture_steps<CudaGraphs>(stream_, [&] { launch(len, nullptr); });
   launched_ = before;  // captured, not run
-  cudaError_t e = cudaStreamEndCapture(stream_, &g);
-  if (!ok && e == cudaSuccess) e = cudaErrorStreamCaptureInvalidated;
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&graph_exec_, g, 0);
-  if (g) cudaGraphDestroy(g);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    graph_exec_ = nullptr;
-    graph_failed_ = true;
-    return;
-  }
+  graph_failed_ = !graph_exec_;
   graph_len_ = len;
 }
 
