@@ -40,3 +40,26 @@ struct CudaGraphs {
 }  // namespace tf
 
 #define CU(call) ::tf::cuda_check((call), #call, __FILE__, __LINE__)
+
+namespace tf {
+
+// Makes a device current for a call that launches and whose caller may have
+// another one current, and puts that back.
+class DeviceGuard {
+ public:
+  explicit DeviceGuard(int device) {
+    CU(cudaGetDevice(&before_));
+    if (before_ != device) CU(cudaSetDevice(device));
+    else before_ = -1;
+  }
+  ~DeviceGuard() {
+    if (before_ >= 0) cudaSetDevice(before_);
+  }
+  DeviceGuard(const DeviceGuard&) = delete;
+  DeviceGuard& operator=(const DeviceGuard&) = delete;
+
+ private:
+  int before_ = -1;
+};
+
+}  // namespace tf

@@ -2124,6 +2124,7 @@ void TetSim::probe_points(double* xyz, uint64_t* cells, size_t cap) const {
 
 void TetSim::get_state(double* U, double* B, double* F) {
   if (group_) return group_->get_state(0, U, B, F);
+  const DeviceGuard on(opt_.device);  // the export launches a kernel
   // dga: renumbered and widened on the GPU, one field at a time
   auto get = [&](const void* v, const int32_t* where, size_t n, double* out) {
     if (!out || !n) return;
