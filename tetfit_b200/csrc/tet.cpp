@@ -1831,7 +1831,10 @@ void TetSim::alloc_and_upload() {
   d.nE = (int)NE;
   d.nF = (int)NF;
   d.dt = dt_;
-  d.U = zeros(NE); d.F = zeros(NF); d.B = zeros(NF); d.cu = zeros(NF); d.cf = zeros(NE);
+  d.U = zeros(NE); d.F = zeros(NF);
+  // what the SELL-32 matrices multiply: a zero behind the last value for their
+  // padding entries (0 times an infinite value would be NaN)
+  d.B = zeros(NF + 1); d.cu = zeros(NF + 1); d.cf = zeros(NE + 1);
   d.I = zeros(NE); d.cb = zeros(NE);
   // device numbering: chunks of 4096 rows, rows of one form (the same column
   // offsets) side by side within them, as in the group engine's layout
@@ -1886,7 +1889,7 @@ void TetSim::alloc_and_upload() {
           for (int l = 0; l < 32; l++) {
             const int64_t q = ptr[s] + 32 * j + l;
             const bool real = j < nr[l];
-            const int32_t c = real || nr[l] ? col_new[m.col[k0[l] + (real ? j : 0)]] : 0;
+            const int32_t c = real ? col_new[m.col[k0[l] + j]] : (int32_t)col_new.size();
             const double v = real ? m.val[k0[l] + j] : 0.0;
             if (values) {
               col[q] = c;

@@ -16,7 +16,8 @@
 namespace tf {
 
 // 32-row slices: entry j of row i at ptr[i / 32] + 32 j + i % 32.  Padding
-// entries have value 0 and the row's first column (C^T: kNoFace).
+// entries have value 0 and the column behind the last, where the multiplied
+// vectors (cf, cu, B) hold a zero (C^T: kNoFace).
 struct TetSell {
   const int64_t* ptr = nullptr;
   const int32_t* col = nullptr;
