@@ -1255,11 +1255,18 @@ template <typename T>
 int group_cg_blocks(int device, int S, size_t* smem) {
   const size_t sm = cg_smem<T>(S);
   if (smem) *smem = sm;
-  int sms = 0, a = 0, b = 0;
+  int sms = 0, most = 0, a = 0, b = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (cudaFuncSetAttribute(grp_cg<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess ||
-      cudaFuncSetAttribute(grp_cg<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
-    return 0;
+  cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  // the limit is the kernel's, for every group on the device: as much as there
+  // is, not this group's need, which may be less than another's
+  auto allow = [&](auto kernel) {
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess || sm + fa.sharedSizeBytes > (size_t)most) return false;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                most - (int)fa.sharedSizeBytes) == cudaSuccess;
+  };
+  if (!allow(grp_cg<T, true>) || !allow(grp_cg<T, false>)) return 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, grp_cg<T, true>, cg_threads<T>(), sm);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, grp_cg<T, false>, cg_threads<T>(), sm);
   return (a < b ? a : b) * sms;
