@@ -181,7 +181,7 @@ void TetGroup::build(std::vector<TetSim*>& sims, bool release_host) {
     // 4096 rows keep what a block gathers close together (40^3 FP32, a solve:
     // one chunk 316 us, 16384 rows 272, 4096 264, 1024 276); grp_cg ran 1 %
     // slower with them.
-    const int32_t chunk = resident_slices <= (int64_t)sms * kCgResidentWarps * kCgResidentRows ? 4096 : INT32_MAX;
+    const int chunk_bits = resident_slices <= (int64_t)sms * kCgResidentWarps * kCgResidentRows ? 12 : 31;
     std::vector<int32_t> old_of_new(nf), pos(nf), cls(nf);
     auto alen_old = [&](int32_t k) { return t.A_.ptr[k + 1] - t.A_.ptr[k]; };
     {
@@ -196,7 +196,7 @@ void TetGroup::build(std::vector<TetSim*>& sims, bool release_host) {
     std::iota(old_of_new.begin(), old_of_new.end(), 0);
     parallel_stable_sort(old_of_new.begin(), old_of_new.end(), opt_.setup_threads,
                          [&](int32_t a, int32_t b) {
-                           const int32_t ca = a / chunk, cb = b / chunk;
+                           const int32_t ca = a >> chunk_bits, cb = b >> chunk_bits;
                            return ca != cb ? ca < cb : cls[a] < cls[b];
                          });
     for (int64_t p = 0; p < nf; p++) pos[old_of_new[p]] = (int32_t)p;
