@@ -1,13 +1,15 @@
-"""Scenes of more coefficient classes than the class kernels' tables hold, on a
-grid that the march kernels take and on one that the autotuner measures,
-against the node-slot kernels bit for bit."""
+"""Routes of a FIT step against the node-slot kernels bit for bit: scenes of more
+coefficient classes than the class kernels' tables hold, on a grid that the march
+kernels take and on one that the autotuner measures; the class kernels on both
+sides of the limit of their programmatic launches."""
 import os
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
 
 import tetfit_b200 as tb
-from tetfit_b200.cases import FitCase, Sphere, write_fit_cavity
+from tetfit_b200.cases import FitCase, Sphere, random_spheres, write_fit_cavity
 
 pytestmark = pytest.mark.gpu
 
@@ -48,5 +50,17 @@ def test_more_classes_than_the_tables_hold(tmp_path, product_lib, n, steps, prec
     got, variant = results(script, steps, n < 100, precision=precision)
     ref, _ = results(script, steps, n < 100, precision=precision, fit_variant=1)
     assert variant == 2 * 9 if n < 100 else (variant % 8 != 5 and variant // 8 != 5)
+    for a, b in zip(got, ref):
+        assert np.array_equal(a, b)
+
+
+# launches of up to 2,048 blocks are programmatic, in FP64 to about 97^3 cells (the
+# two runs' host set-up, most of the test's time, goes side by side)
+@pytest.mark.parametrize("n", [95, 100])
+def test_class_steps_on_both_sides_of_the_programmatic_limit(tmp_path, product_lib, n):
+    script = write_fit_cavity(str(tmp_path), FitCase(n=n, steps=20, spheres=random_spheres(20, seed=n)))
+    with ThreadPoolExecutor(2) as pool:
+        (got, variant), (ref, node) = pool.map(lambda v: results(script, 20, True, fit_variant=v), (0, 1))
+    assert variant == 5 * 9 and node == 0
     for a, b in zip(got, ref):
         assert np.array_equal(a, b)
