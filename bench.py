@@ -387,10 +387,10 @@ def precision_report(script, device, steps=400, every=100):
 
 
 # DRAM traffic of the FIT class kernels measured by ncu (one launch each of
-# the 256^3 scene, state 607 MB > L2, 32 x 4 blocks): fit_e_class 689.7 MB
-# against 709.4 MB algorithmic, fit_h_class 697.6 MB against 708.2 MB.  The ratio is per byte
-# (one plane per block, the same re-use at every size), reported for the
-# dominant kernel as ratio x its algorithmic bytes.
+# the 256^3 scene, state 607 MB > L2): fit_e_class 716.1 MB against 709.4 MB
+# algorithmic, fit_h_class 701.0 MB against 708.2 MB.  The ratio is per byte
+# (16-byte packs in the arrays' order, neighbouring rows and planes found in L2),
+# reported for the dominant kernel as ratio x its algorithmic bytes.
 FIT_DRAM_OVER_ALGORITHMIC = {("fit_e_class", 4): 1.009, ("fit_h_class", 4): 0.990}
 FIT_TRAFFIC_NOTE = "ncu DRAM bytes / algorithmic bytes of the kernel at 256^3, times this launch's algorithmic bytes"
 

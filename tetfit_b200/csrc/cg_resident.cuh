@@ -45,7 +45,7 @@ __device__ __forceinline__ double cg_warp_sum(double v) {
 // The blocks [first, first + count) of one system.  Every block has a box per
 // value with a record from each block of its system: a record has one reader,
 // which keeps the pollers out of one another's way (148 blocks reading one set
-// of 148 records wait 3 to 5 us for one another in L2, with boxes 2 to 3).
+// of 148 records wait 3.4 to 5.4 us for one another in L2, with boxes 2.3 to 3.3).
 // box[parity][value][block][producer]
 //
 // With clusters of `cluster` blocks (one system a launch, at most 32 clusters)

@@ -1276,19 +1276,19 @@ __global__ void __launch_bounds__(256) fit_h_coef(FitGrid<T> g, int* step_counte
 }
 
 // ------------------------------------------------------- coefficient classes
-// The class variant makes a leapfrog step of two launches.  fit_e_class: the
-// special edges' blocks first (their source chain is the longest), blocks
-// that set the probes' face values aside, then the interior edges.
-// fit_h_class: the probes' blocks, the boundary flux sum, then the faces.
+// The class variant makes a leapfrog step of two launches, each with blocks of
+// other work spread among its interior ones (extra_block).  fit_e_class: the
+// interior edges, the special edges, and blocks that set the probes' face values
+// aside.  fit_h_class: the faces, the probes and the boundary flux sum.
 // Nothing in a launch reads what the launch writes: the E half reads F and
 // each edge's own U, the H half reads U and each face's own F, an edge has one
 // writer (the special edges carry kNoClass, which the interior part leaves
 // alone), and the probes read the faces' old values from the copy.
 //
-// Bounds: launch latency on small grids, DRAM on large ones (256^3 FP32: the
-// E half moves 0.66 GB, the H half 0.66 GB; 135 and 121 us, 0.75 and 0.84 of
-// the measured copy bandwidth; one slot per thread in five launches took 158
-// and 162 us, a 24^3 FP64 step 64 us against 6).  Three blocks of 256 an SM
+// Bounds: launch latency on small grids, DRAM on large ones (256^3 FP32: 0.709
+// and 0.708 GB of state and classes in 130 and 119 us, 0.83 and 0.91 of the
+// measured copy bandwidth; one slot per thread in five launches took 159 and
+// 163 us, a 24^3 FP64 step 64 us against 6).  Three blocks of 256 an SM
 // leave room for every load of a thread in flight at once (80 registers);
 // four (64 registers) spill and ran 20 % slower at 256^3.
 //

@@ -1765,8 +1765,9 @@ void TetSim::build_sources() {
 
 // Rows of a matrix in chunks of 4096, rows whose column offsets (col - row)
 // are the same side by side within a chunk, each form in its own order.  The
-// forms are told apart by a hash of the offsets; equal hashes of different
-// forms would only mix them.
+// forms are told apart by an FNV-1a hash of the offsets (a word at a time, with
+// a shift to mix the upper half in); equal hashes of different forms would only
+// mix them.
 static std::vector<int32_t> stencil_order(const HostCsr& m, int threads) {
   const int64_t n = (int64_t)m.ptr.size() - 1;
   std::vector<uint64_t> form(n);
